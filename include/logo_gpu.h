@@ -208,8 +208,9 @@ typedef struct logo_instance {
     uint64_t seed; /* kick PRNG seed (SplitMix64 state) */
 } logo_instance;
 
-/* Tile shape of the batched kernel: rows per thread, threads per CTA (one
- * CTA per instance), columns per warp tile. */
+/* Shape of the batched kernel: threads per CTA (one CTA per instance).  Rows
+ * per thread and columns per tile are part of a shape's name only (the sweep
+ * goes over cities and their neighbours, not over tiles of pairs). */
 typedef struct logo_batch_shape {
     int rows_per_thread;
     int threads_per_cta;
@@ -306,7 +307,7 @@ typedef struct logo_server logo_server;
 typedef struct logo_server_opts {
     int device;
     uint64_t mem_budget;    /* device bytes for resident requests; 0 = 2 GiB */
-    uint32_t max_slots;     /* requests with n <= LOGO_BATCH_MAX_N in flight; 0 = SMs x occupancy */
+    uint32_t max_slots;     /* requests with n <= LOGO_BATCH_MAX_N in flight; 0 = 4 x SMs */
     uint32_t max_large;     /* larger requests in flight; 0 = 2 */
     uint32_t kicks;         /* ILS kicks per request after its first descent */
     int kick_kind;          /* LOGO_KICK_* */

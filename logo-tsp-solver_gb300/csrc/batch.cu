@@ -7,7 +7,7 @@
 // (or one per pthread, ILSGlobalSolverMT.cpp:86-195) and crosses the PCIe bus
 // three times per move.  The per-instance algorithm is the reference's:
 //   sweep     ≙ CPUSolver::optimizeStep loop order, per-edge nint
-//               (src/solvers/cpuSolver.cpp:188-230) -- sweep_core.cuh
+//               (src/solvers/cpuSolver.cpp:188-230) -- near_tour.cuh
 //   move      ≙ rotate + reverse (src/solvers/twoOptLocalSolver.cpp:41-48)
 //   descent   ≙ TwoOptLocalSolver::optimize (twoOptLocalSolver.cpp:22-64)
 //   ILS       ≙ ILSGlobalSolverSequential::optimize with a kick count
@@ -18,20 +18,16 @@
 //
 // Scheduling: a global atomic work queue over instances sorted by descending
 // n (longest first); each CTA pops the next instance when it finishes one.
-// In shared memory the tour is permuted in place: a move
-// new = old[i..c) ++ rev(old[0..i)) ++ rev(old[c..n)) is the three reversals
-// rev[i,c) + rev[c,n) (disjoint, one phase), then rev[0,c).
+// The tour, its neighbour lists and the sweep are those of near_tour.cuh.
 #include <cstdint>
 
 #include "batch_internal.h"
 #include "logo_device.cuh"
-#include "cta_tour.cuh"
-#include "sweep_core.cuh"
+#include "near_tour.cuh"
 
 namespace logo {
 
-static_assert((kBatchMaxN - 3 + kWin7 - 1) / kWin7 <= kCtaWindows,
-              "the CTA sweep's window statistics cover the largest instance");
+static_assert(kBatchMaxN <= kNearMaxN, "one CTA holds the largest instance");
 
 namespace {
 
@@ -47,7 +43,7 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned int* p) {
 // again after its next descent.
 template <int NT>
 __device__ void publish_best(SharedBest* g, uint32_t* tours, const uint32_t* bestr, uint32_t n,
-                             unsigned long long best_len, unsigned int* flag) {
+                             unsigned long long best_len, NearShared<NT>& S) {
     if (threadIdx.x == 0) {
         unsigned int f = 0;
         if (best_len < *(volatile unsigned long long*)&g->best_len &&
@@ -60,10 +56,10 @@ __device__ void publish_best(SharedBest* g, uint32_t* tours, const uint32_t* bes
                 atomicExch(&g->lock, 0u);
             }
         }
-        *flag = f;
+        S.flag = f;
     }
     __syncthreads();
-    if (*flag) {
+    if (S.flag) {
         uint32_t* t = tours + g->off;
         for (uint32_t k = threadIdx.x; k < n; k += NT) t[k] = bestr[k];
         __threadfence();
@@ -78,40 +74,35 @@ __device__ void publish_best(SharedBest* g, uint32_t* tours, const uint32_t* bes
     __syncthreads();
 }
 
-// Loads the group's best tour into route / Q (coordinates; the caller
-// recomputes edges) when one is published that is no longer than this
-// replica's best; false (route / Q possibly overwritten) when there is none
-// or it changed while being read.
+// Copies the group's best tour into T.id (the caller places it) when one is
+// published that is no longer than this replica's best; false (T.id possibly
+// overwritten) when there is none or it changed while being read.
 template <int NT>
-__device__ bool adopt_best(SharedBest* g, const uint32_t* tours, uint32_t* route,
-                           OrderedCity* Q, const float2* xy, uint32_t n,
-                           unsigned long long best_len, unsigned int* flag, unsigned int* s1) {
+__device__ bool adopt_best(SharedBest* g, const uint32_t* tours, const NearTour& T,
+                           unsigned long long best_len, NearShared<NT>& S) {
     if (threadIdx.x == 0) {
         const unsigned int q = ld_acquire_u32(&g->seq);
         const unsigned long long gl = *(volatile unsigned long long*)&g->best_len;
-        *s1 = q;
-        *flag = !(q & 1u) && gl != ~0ull && gl <= best_len;
+        S.seq = q;
+        S.flag = !(q & 1u) && gl != ~0ull && gl <= best_len;
     }
     __syncthreads();
-    if (!*flag) {
+    if (!S.flag) {
         __syncthreads();
         return false;
     }
     const uint32_t* t = tours + g->off;
-    for (uint32_t k = threadIdx.x; k < n; k += NT) {
+    for (uint32_t k = threadIdx.x; k < T.n; k += NT) {
         const uint32_t c = __ldcg(t + k);
-        route[k] = c < n ? c : 0u;
-        const float2 p = xy[route[k]];
-        Q[k].x = p.x;
-        Q[k].y = p.y;
+        T.id[k] = (uint16_t)(c < T.n ? c : 0u);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        *flag = ld_acquire_u32(&g->seq) == *s1;
+        S.flag = ld_acquire_u32(&g->seq) == S.seq;
     }
     __syncthreads();
-    const bool ok = *flag;
+    const bool ok = S.flag;
     __syncthreads();
     return ok;
 }
@@ -533,16 +524,13 @@ __global__ void __launch_bounds__(kMfThreads)
     }
 }
 
-template <int R, int NT, int TC>
-__global__ void __launch_bounds__(NT)
+template <int NT>
+__global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
     batch_kernel(BatchArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ CtaShared<NT> S;
-    __shared__ CtaWindows W;
-    __shared__ unsigned int share_flag, share_seq;
-    OrderedCity* Q = reinterpret_cast<OrderedCity*>(smem_raw);
-    uint32_t* route = reinterpret_cast<uint32_t*>(smem_raw + sizeof(OrderedCity) * A.max_n);
-    uint32_t* bestr = route + A.max_n;
+    __shared__ NearShared<NT> S;
+    uint32_t parity = 0;
+    near_init<NT>(S);
 
     for (;;) {
         if (threadIdx.x == 0) S.idx = atomicAdd(A.queue, 1u);
@@ -555,26 +543,23 @@ __global__ void __launch_bounds__(NT)
         const uint32_t n = I.n;
         const float2* xy = A.coords + I.off;
         uint32_t* rio = A.routes + I.off;
+        NearTour T = near_carve(smem_raw, n);
 
-        // load (or build) the start tour, its ordered coordinates and edge lengths
-        if (A.start == kStartNN) nn_tour_cta<NT>(xy, n, route, bestr);
-        for (uint32_t k = threadIdx.x; k < n; k += NT) {
-            const uint32_t c = A.start == kStartNN ? route[k] : rio[k];
-            const float2 p = xy[c];
-            route[k] = c;
-            bestr[k] = c;
-            OrderedCity o;
-            o.x = p.x;
-            o.y = p.y;
-            o.e = 0.f;
-            o.pad = 0.f;
-            Q[k] = o;
+        // load (or build) the start tour; rio holds the best tour from here on
+        if (A.start == kStartNN) {  // the list area holds the builder's two arrays
+            uint32_t* route = reinterpret_cast<uint32_t*>(T.nbr);
+            nn_tour_cta<NT>(xy, n, route, route + n);
+            for (uint32_t k = threadIdx.x; k < n; k += NT) {
+                rio[k] = route[k];
+                T.id[k] = (uint16_t)route[k];
+            }
+        } else {
+            for (uint32_t k = threadIdx.x; k < n; k += NT) T.id[k] = (uint16_t)rio[k];
         }
-        if (threadIdx.x == 0) fill_tile_table<R, TC>(S, n);
         __syncthreads();
-        recompute_edges<NT>(Q, n);
-        __syncthreads();
-        const unsigned long long start_len = tour_length<NT>(S, Q, n);
+        near_build<NT>(T, S, xy);
+        near_place<NT>(T, xy);
+        const unsigned long long start_len = near_length<NT>(T, S);
         unsigned long long best_len = start_len;
         unsigned long long moves = 0, sweeps = 0;
         uint32_t accepted = 0, status = 0;
@@ -585,9 +570,8 @@ __global__ void __launch_bounds__(NT)
             // descent
             unsigned long long dm = 0;
             for (;;) {
-                window_stats_cta<NT>(W, Q, n);
-                __syncthreads();
-                const unsigned long long key = sweep_boxed<R, NT, TC>(S, W, Q, n, I.margin);
+                const unsigned long long key = near_sweep<NT>(T, S, parity);
+                parity ^= 1u;
                 ++sweeps;
                 if (key == kNoMove) break;
                 const uint32_t p = key_i(key), q = key_j(key);
@@ -595,7 +579,7 @@ __global__ void __launch_bounds__(NT)
                     status |= kErrBadKey;
                     break;
                 }
-                rotate_reverse<NT>(Q, route, n, p, q);
+                near_move<NT>(T, p, q);
                 ++moves;
                 if (++dm >= move_cap) {
                     status |= kErrMoveLimit;
@@ -605,30 +589,21 @@ __global__ void __launch_bounds__(NT)
             if (status) break;
             // accept (strictly shorter) or go back: to the replica's own best
             // tour, or in a multi-start group to the group's best
-            const unsigned long long len = tour_length<NT>(S, Q, n);
+            const unsigned long long len = near_length<NT>(T, S);
             SharedBest* grp = I.group != kNoGroup ? A.shared + I.group : nullptr;
             if (len < best_len) {
                 best_len = len;
                 ++accepted;
-                for (uint32_t k = threadIdx.x; k < n; k += NT) bestr[k] = route[k];
+                for (uint32_t k = threadIdx.x; k < n; k += NT) rio[k] = T.id[T.slot(k)];
                 __syncthreads();
             } else {
-                const bool adopted = grp && adopt_best<NT>(grp, A.shared_tours, route, Q, xy, n,
-                                                           best_len, &share_flag, &share_seq);
-                if (!adopted) {
-                    for (uint32_t k = threadIdx.x; k < n; k += NT) {
-                        const uint32_t c = bestr[k];
-                        route[k] = c;
-                        const float2 p = xy[c];
-                        Q[k].x = p.x;
-                        Q[k].y = p.y;
-                    }
-                }
+                const bool adopted = grp && adopt_best<NT>(grp, A.shared_tours, T, best_len, S);
+                if (!adopted)
+                    for (uint32_t k = threadIdx.x; k < n; k += NT) T.id[k] = (uint16_t)rio[k];
                 __syncthreads();
-                recompute_edges<NT>(Q, n);
+                near_place<NT>(T, xy);
             }
-            __syncthreads();
-            if (grp) publish_best<NT>(grp, A.shared_tours, bestr, n, best_len, &share_flag);
+            if (grp) publish_best<NT>(grp, A.shared_tours, rio, n, best_len, S);
             if (it == A.kicks) break;
             // kick: every thread draws the same numbers from the same state
             if (A.kick_kind == 1) {
@@ -639,15 +614,14 @@ __global__ void __launch_bounds__(NT)
                 if (c1 < c0) { t = c0; c0 = c1; c1 = t; }
                 if (c2 < c1) { t = c1; c1 = c2; c2 = t; }
                 if (c1 < c0) { t = c0; c0 = c1; c1 = t; }
-                double_bridge<NT>(Q, route, n, c0, c1, c2);
+                near_double_bridge<NT>(T, c0, c1, c2);
             } else {
                 uint32_t a = uniform_below(rng, n);
                 uint32_t b = uniform_below(rng, n);
                 if (b < a) { const uint32_t t = a; a = b; b = t; }
-                rotate_reverse<NT>(Q, route, n, a, b);
+                near_move<NT>(T, a, b);
             }
         }
-        for (uint32_t k = threadIdx.x; k < n; k += NT) rio[k] = bestr[k];
         if (threadIdx.x == 0) {
             BatchResult r;
             r.start_length = start_len;
@@ -666,29 +640,28 @@ __global__ void __launch_bounds__(NT)
 
 }  // namespace
 
-size_t batch_smem_bytes(uint32_t max_n) {
-    return (size_t)max_n * (sizeof(OrderedCity) + 2 * sizeof(uint32_t));
-}
+size_t batch_smem_bytes(uint32_t max_n) { return near_layout(max_n).bytes; }
 
-template <int R, int NT, int TC>
+template <int NT>
 static cudaError_t launch_batch_t(const BatchArgs& A, int grid, cudaStream_t s,
                                   int* occupancy) {
     const size_t smem = batch_smem_bytes(A.max_n);
     if (occupancy) {
         // the attribute is set here, outside any stream capture, and for the
         // largest instance (it is shared by every batch object in the process)
-        const size_t cap = batch_smem_bytes(kBatchMaxN);
-        cudaError_t e = cudaFuncSetAttribute(batch_kernel<R, NT, TC>,
+        cudaError_t e = cudaFuncSetAttribute(batch_kernel<NT>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(cap > 48 * 1024 ? cap : 48 * 1024));
+                                             (int)batch_smem_bytes(kBatchMaxN));
         if (e != cudaSuccess) return e;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, batch_kernel<R, NT, TC>,
-                                                             NT, smem);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, batch_kernel<NT>, NT, smem);
     }
-    batch_kernel<R, NT, TC><<<grid, NT, smem, s>>>(A);
+    batch_kernel<NT><<<grid, NT, smem, s>>>(A);
     return cudaGetLastError();
 }
 
+// The shapes a caller may ask for: threads per CTA is what is compiled for;
+// rows per thread and tile columns belonged to sweeps over tiles of pairs and
+// are accepted as names.
 #define LOGO_BATCH_SHAPES(X) \
     X(2, 128, 64)            \
     X(2, 256, 64)            \
@@ -701,7 +674,7 @@ static cudaError_t launch_batch_t(const BatchArgs& A, int grid, cudaStream_t s,
 cudaError_t launch_batch(const BatchArgs& A, const BatchShape& sh, int grid, cudaStream_t s,
                          int* occupancy) {
 #define X(r, nt, tc) \
-    if (sh.R == r && sh.NT == nt && sh.TC == tc) return launch_batch_t<r, nt, tc>(A, grid, s, occupancy);
+    if (sh.R == r && sh.NT == nt && sh.TC == tc) return launch_batch_t<nt>(A, grid, s, occupancy);
     LOGO_BATCH_SHAPES(X)
 #undef X
     return cudaErrorInvalidValue;

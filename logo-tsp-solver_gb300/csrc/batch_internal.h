@@ -16,9 +16,7 @@ struct BatchInstance {
     unsigned long long off;   // first city of this instance in coords / routes
     unsigned long long seed;  // kick PRNG state
     uint32_t n;
-    float margin;             // filter margin for this instance's coordinates
     uint32_t group;           // shared-best group (multi-start), or kNoGroup
-    uint32_t pad;
 };
 
 // Best tour shared by the replicas of one multi-start group.  A writer holds
@@ -60,9 +58,9 @@ struct BatchArgs {
 };
 
 struct BatchShape {
-    int R;   // rows per thread
+    int R;   // rows per thread (a name only, see LOGO_BATCH_SHAPES in batch.cu)
     int NT;  // threads per CTA
-    int TC;  // columns per warp tile
+    int TC;  // columns per warp tile (a name only)
 };
 
 size_t batch_smem_bytes(uint32_t max_n);

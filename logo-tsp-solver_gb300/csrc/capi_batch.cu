@@ -28,8 +28,11 @@ int bucket_of(uint32_t n) {
     return kBuckets - 1;
 }
 
+// A sweep's latency falls with the threads it is spread over (n = 1,987 from a
+// random tour on one GB300: 68 us a sweep with 128 threads, 39 with 256, 25
+// with 512); below a few hundred cities more threads find nothing to do.
 const BatchShape kDefaultShape[kBuckets] = {
-    {2, 128, 64}, {2, 128, 64}, {4, 256, 64}, {4, 256, 128}, {4, 256, 128}};
+    {2, 128, 64}, {4, 256, 64}, {4, 512, 128}, {4, 512, 128}, {4, 512, 128}};
 
 thread_local std::string g_batch_err;
 
@@ -54,6 +57,10 @@ struct logo_batch {
     SharedBest* d_shared = nullptr;     // multi-start: the group's best (one group)
     uint32_t* d_shared_tours = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // launch groups after the first are captured on these, as branches of the
+    // run's graph (made on first use)
+    cudaStream_t side[8] = {};
+    cudaEvent_t forked = nullptr, joined[8] = {};
     BatchShape table[kBuckets];
     int sms = 0;
     std::string gpu;
@@ -95,6 +102,11 @@ void free_batch(logo_batch* b) {
     if (b->h_inst) cudaFreeHost(b->h_inst);
     if (b->h_order) cudaFreeHost(b->h_order);
     if (b->h_res) cudaFreeHost(b->h_res);
+    for (int k = 0; k < 8; ++k) {
+        if (b->side[k]) cudaStreamDestroy(b->side[k]);
+        if (b->joined[k]) cudaEventDestroy(b->joined[k]);
+    }
+    if (b->forked) cudaEventDestroy(b->forked);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -156,9 +168,7 @@ logo_status pack(logo_batch* b, const logo_instance* in, uint32_t count, bool gi
         d.off = off;
         d.seed = I.seed;
         d.n = I.n;
-        d.margin = filter_margin(diag);
         d.group = kNoGroup;
-        d.pad = 0;
         b->h_inst[k] = d;
         off += I.n;
     }
@@ -239,8 +249,18 @@ logo_status run(logo_batch* b, const logo_instance* in, uint32_t count,
     BCK(b, cudaMemcpyAsync(b->d_order, b->h_order, sizeof(uint32_t) * count,
                            cudaMemcpyHostToDevice, b->stream));
     BCK(b, cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int) * 8, b->stream));
-    // one CUDA graph per run: every group's persistent launch back to back
+    // one CUDA graph per run: the groups' persistent launches side by side (the
+    // one with the largest instances first), so that a group's CTAs start where
+    // another's last instances leave SMs free
     std::vector<int> grids(groups.size());
+    if (groups.size() > 8) return bfail(b, LOGO_ERR_CUDA, "more launch groups than shapes");
+    if (groups.size() > 1 && !b->forked)
+        BCK(b, cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming));
+    for (size_t gi = 1; gi < groups.size(); ++gi) {
+        if (!b->side[gi]) BCK(b, cudaStreamCreateWithFlags(&b->side[gi], cudaStreamNonBlocking));
+        if (!b->joined[gi])
+            BCK(b, cudaEventCreateWithFlags(&b->joined[gi], cudaEventDisableTiming));
+    }
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         BatchArgs A{};
         A.max_n = groups[gi].max_n;
@@ -262,7 +282,8 @@ logo_status run(logo_batch* b, const logo_instance* in, uint32_t count,
     if (o.start == LOGO_START_MF)
         ce = launch_mf_start(b->d_coords, b->d_routes, b->d_inst, b->d_order, count, max_n_all,
                              b->sms, b->stream);
-    for (size_t gi = 0; gi < groups.size() && ce == cudaSuccess && gi < 8; ++gi) {
+    if (ce == cudaSuccess && groups.size() > 1) ce = cudaEventRecord(b->forked, b->stream);
+    for (size_t gi = 0; gi < groups.size() && ce == cudaSuccess; ++gi) {
         BatchArgs A;
         A.coords = b->d_coords;
         A.routes = b->d_routes;
@@ -277,10 +298,15 @@ logo_status run(logo_batch* b, const logo_instance* in, uint32_t count,
         A.shared = share ? b->d_shared : nullptr;
         A.shared_tours = share ? b->d_shared_tours : nullptr;
         A.start = o.start == LOGO_START_NN ? kStartNN : kStartGiven;
-        ce = launch_batch(A, groups[gi].shape, grids[gi], b->stream, nullptr);
+        const cudaStream_t gs = gi == 0 ? b->stream : b->side[gi];
+        if (gi > 0) ce = cudaStreamWaitEvent(gs, b->forked, 0);
+        if (ce == cudaSuccess) ce = launch_batch(A, groups[gi].shape, grids[gi], gs, nullptr);
+        if (ce == cudaSuccess && gi > 0) ce = cudaEventRecord(b->joined[gi], gs);
     }
+    for (size_t gi = 1; gi < groups.size() && ce == cudaSuccess; ++gi)
+        ce = cudaStreamWaitEvent(b->stream, b->joined[gi], 0);
     cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
-    if (ce != cudaSuccess || ee != cudaSuccess || groups.size() > 8) {
+    if (ce != cudaSuccess || ee != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return bfail(b, LOGO_ERR_CUDA, std::string("batch capture: ") +
                                            cudaGetErrorString(ce != cudaSuccess ? ce : ee));
@@ -522,6 +548,9 @@ logo_status logo_batch_autotune(logo_batch* b, const logo_instance* sample, uint
         BatchShape best = b->table[bk];
         std::vector<uint64_t> ref_len;
         for (int si = 0; si < nshapes; ++si) {
+            bool timed = false;  // shapes with the same threads per CTA are one kernel
+            for (int k = 0; k < si; ++k) timed |= shapes[k].NT == shapes[si].NT;
+            if (timed) continue;
             for (size_t k = 0; k < sub.size(); ++k) {
                 std::copy(routes[k].begin(), routes[k].end(), const_cast<uint32_t*>(sub[k].route));
             }

@@ -49,7 +49,6 @@ struct Req {
     uint64_t id = 0;
     uint32_t n = 0;
     uint64_t seed = 0;
-    float margin = 0.f;
     std::vector<logo_xy> xy;
     std::vector<uint32_t> route;  // start tour, then the result
     ReqState state = kPending;
@@ -270,7 +269,6 @@ void admit(logo_server* s) {
                 st.phase = kServeInit;
                 st.kicks_total = s->opts.kicks;
                 st.kick_kind = s->opts.kick_kind;
-                st.margin = r.margin;
                 cudaMemcpyAsync(s->d_slots + slot, &st, sizeof(ServeSlot), cudaMemcpyHostToDevice,
                                 s->stream);
                 ok = true;
@@ -428,7 +426,9 @@ logo_status logo_server_create(const logo_server_opts* o, logo_server** out) {
         launch_serve_round(A, 0, nullptr, &s->occ);
         if (s->occ < 1) s->occ = 1;
     }
-    if (!s->opts.max_slots) s->opts.max_slots = (uint32_t)(s->occ * s->sms * 2);
+    // resident tours cost little and rounds take the slots largest first: four
+    // a SM, whatever the shared memory of the largest size allows at once
+    if (!s->opts.max_slots) s->opts.max_slots = (uint32_t)(s->sms * 4);
     s->arena_cap = s->opts.mem_budget / kSmallBytesPerCity;
     s->arena.reset(s->arena_cap);
     s->slot_req.assign(s->opts.max_slots, -1);
@@ -486,7 +486,6 @@ logo_status logo_server_submit(logo_server* s, const logo_xy* coords, uint32_t n
     Req r;
     r.n = n;
     r.seed = seed;
-    r.margin = filter_margin(diag);
     r.xy.assign(coords, coords + n);
     r.route.assign(route, route + n);
     r.large = n > kBatchMaxN;

@@ -17,24 +17,27 @@
 // slots share a round, so a request's result is the same alone and in any mix.
 #include <cstdint>
 
-#include "cta_tour.cuh"
-#include "logo_device.cuh"
 #include "batch_internal.h"
+#include "logo_device.cuh"
+#include "near_tour.cuh"
 #include "serve_internal.h"
-#include "sweep_core.cuh"
 
 namespace logo {
 
 namespace {
 
-template <int R, int NT, int TC>
-__global__ void __launch_bounds__(NT) serve_round_kernel(ServeArgs A) {
+// Pair evaluations charged per city and sweep: a sweep looks at a few listed
+// neighbours of each city (near_tour.cuh counts them), 16 is what its lists
+// hold.
+constexpr unsigned long long kServePairsPerCity = 16;
+
+template <int NT>
+__global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
+    serve_round_kernel(ServeArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ CtaShared<NT> S;
-    __shared__ CtaWindows W;
-    OrderedCity* Q = reinterpret_cast<OrderedCity*>(smem_raw);
-    uint32_t* route = reinterpret_cast<uint32_t*>(smem_raw + sizeof(OrderedCity) * A.max_n);
-    uint32_t* bestr = route + A.max_n;
+    __shared__ NearShared<NT> S;
+    uint32_t parity = 0;
+    near_init<NT>(S);
 
     for (;;) {
         if (threadIdx.x == 0) S.idx = atomicAdd(A.queue, 1u);
@@ -49,40 +52,31 @@ __global__ void __launch_bounds__(NT) serve_round_kernel(ServeArgs A) {
         const float2* xy = A.coords + st.off;
         uint32_t* rio = A.route + st.off;
         uint32_t* bio = A.best + st.off;
+        NearTour T = near_carve(smem_raw, n);
 
-        // load the resident tour (and best tour) into shared memory
+        // load the resident tour into shared memory (the best one stays in the arena)
         for (uint32_t k = threadIdx.x; k < n; k += NT) {
             const uint32_t c = rio[k];
-            route[k] = c;
-            bestr[k] = (st.phase == kServeInit) ? c : bio[k];
-            const float2 p = xy[c];
-            OrderedCity o;
-            o.x = p.x;
-            o.y = p.y;
-            o.e = 0.f;
-            o.pad = 0.f;
-            Q[k] = o;
+            T.id[k] = (uint16_t)c;
+            if (st.phase == kServeInit) bio[k] = c;
         }
-        if (threadIdx.x == 0) fill_tile_table<R, TC>(S, n);
         __syncthreads();
-        recompute_edges<NT>(Q, n);
-        __syncthreads();
+        near_build<NT>(T, S, xy);
+        near_place<NT>(T, xy);
         if (st.phase == kServeInit) {
-            st.start_len = tour_length<NT>(S, Q, n);
+            st.start_len = near_length<NT>(T, S);
             st.best_len = st.start_len;
             st.phase = kServeDescent;
         }
-        const unsigned long long pairs = n >= 4 ? (unsigned long long)(n - 2) * (n - 3) / 2 : 0;
         const unsigned long long move_cap = 64ull * n * n + 1024;
         unsigned long long spent = 0;
         uint64_t rng = st.rng;
         while (st.phase != kServeDone && spent < A.budget_pairs) {
             if (st.phase == kServeDescent) {
-                window_stats_cta<NT>(W, Q, n);
-                __syncthreads();
-                const unsigned long long key = sweep_boxed<R, NT, TC>(S, W, Q, n, st.margin);
+                const unsigned long long key = near_sweep<NT>(T, S, parity);
+                parity ^= 1u;
                 ++st.sweeps;
-                spent += pairs + n;  // + n: a sweep of a tiny tour still costs work
+                spent += kServePairsPerCity * n;
                 if (key == kNoMove) {
                     st.phase = kServeAccept;
                     continue;
@@ -93,30 +87,24 @@ __global__ void __launch_bounds__(NT) serve_round_kernel(ServeArgs A) {
                     st.phase = kServeDone;
                     break;
                 }
-                rotate_reverse<NT>(Q, route, n, p, q);
+                near_move<NT>(T, p, q);
                 ++st.moves;
                 if (++st.descent_moves >= move_cap) {
                     st.status |= kErrMoveLimit;
                     st.phase = kServeDone;
                 }
             } else {  // kServeAccept: keep if strictly shorter, else revert
-                const unsigned long long len = tour_length<NT>(S, Q, n);
+                const unsigned long long len = near_length<NT>(T, S);
                 if (len < st.best_len) {
                     st.best_len = len;
                     ++st.accepted;
-                    for (uint32_t k = threadIdx.x; k < n; k += NT) bestr[k] = route[k];
-                } else {
-                    for (uint32_t k = threadIdx.x; k < n; k += NT) {
-                        const uint32_t c = bestr[k];
-                        route[k] = c;
-                        const float2 p = xy[c];
-                        Q[k].x = p.x;
-                        Q[k].y = p.y;
-                    }
+                    for (uint32_t k = threadIdx.x; k < n; k += NT) bio[k] = T.id[T.slot(k)];
                     __syncthreads();
-                    recompute_edges<NT>(Q, n);
+                } else {
+                    for (uint32_t k = threadIdx.x; k < n; k += NT) T.id[k] = (uint16_t)bio[k];
+                    __syncthreads();
+                    near_place<NT>(T, xy);
                 }
-                __syncthreads();
                 if (st.kicks_done == st.kicks_total) {
                     st.phase = kServeDone;
                     break;
@@ -129,12 +117,12 @@ __global__ void __launch_bounds__(NT) serve_round_kernel(ServeArgs A) {
                     if (c1 < c0) { t = c0; c0 = c1; c1 = t; }
                     if (c2 < c1) { t = c1; c1 = c2; c2 = t; }
                     if (c1 < c0) { t = c0; c0 = c1; c1 = t; }
-                    double_bridge<NT>(Q, route, n, c0, c1, c2);
+                    near_double_bridge<NT>(T, c0, c1, c2);
                 } else {
                     uint32_t a = uniform_below(rng, n);
                     uint32_t b = uniform_below(rng, n);
                     if (b < a) { const uint32_t t = a; a = b; b = t; }
-                    rotate_reverse<NT>(Q, route, n, a, b);
+                    near_move<NT>(T, a, b);
                 }
                 ++st.kicks_done;
                 st.descent_moves = 0;
@@ -142,11 +130,8 @@ __global__ void __launch_bounds__(NT) serve_round_kernel(ServeArgs A) {
             }
         }
         st.rng = rng;
-        // write the resident state back
-        for (uint32_t k = threadIdx.x; k < n; k += NT) {
-            rio[k] = route[k];
-            bio[k] = bestr[k];
-        }
+        // write the resident state back, in tour order
+        for (uint32_t k = threadIdx.x; k < n; k += NT) rio[k] = T.id[T.slot(k)];
         if (threadIdx.x == 0) A.slots[slot] = st;
         __syncthreads();
     }
@@ -154,22 +139,17 @@ __global__ void __launch_bounds__(NT) serve_round_kernel(ServeArgs A) {
 
 }  // namespace
 
-size_t serve_smem_bytes(uint32_t max_n) {
-    return (size_t)max_n * (sizeof(OrderedCity) + 2 * sizeof(uint32_t));
-}
+size_t serve_smem_bytes(uint32_t max_n) { return near_layout(max_n).bytes; }
 
-// One compiled shape: R = 4 rows per thread, 256 threads, 128-column warp
-// tiles (the fastest measured batched shape for n in [1024, 4096]).
-constexpr int kServeR = 4, kServeNT = 256, kServeTC = 128;
+constexpr int kServeNT = 256;
 
 cudaError_t launch_serve_round(const ServeArgs& A, int grid, cudaStream_t s, int* occupancy) {
     const size_t smem = serve_smem_bytes(A.max_n);
-    auto kern = serve_round_kernel<kServeR, kServeNT, kServeTC>;
+    auto kern = serve_round_kernel<kServeNT>;
     if (occupancy) {
         // for the largest request: the attribute is shared by every server
-        const size_t cap = serve_smem_bytes(kBatchMaxN);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(cap > 48 * 1024 ? cap : 48 * 1024));
+                                             (int)serve_smem_bytes(kBatchMaxN));
         if (e != cudaSuccess) return e;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, kern, kServeNT, smem);
     }

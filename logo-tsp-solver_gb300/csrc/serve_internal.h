@@ -24,7 +24,7 @@ struct ServeSlot {
     uint32_t accepted;
     uint32_t status;                  // kErr* bits
     int kick_kind;
-    float margin;
+    uint32_t pad;
 };
 
 struct ServeArgs {
