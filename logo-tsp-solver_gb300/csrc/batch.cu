@@ -41,9 +41,9 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned int* p) {
 // this replica's best tour to its group if it beats the group's best.  The
 // lock is only tried, never waited for; a replica that finds it taken offers
 // again after its next descent.
-template <int NT>
+template <int NT, typename SH>
 __device__ void publish_best(SharedBest* g, uint32_t* tours, const uint32_t* bestr, uint32_t n,
-                             unsigned long long best_len, NearShared<NT>& S) {
+                             unsigned long long best_len, SH& S) {
     if (threadIdx.x == 0) {
         unsigned int f = 0;
         if (best_len < *(volatile unsigned long long*)&g->best_len &&
@@ -77,9 +77,9 @@ __device__ void publish_best(SharedBest* g, uint32_t* tours, const uint32_t* bes
 // Copies the group's best tour into T.id (the caller places it) when one is
 // published that is no longer than this replica's best; false (T.id possibly
 // overwritten) when there is none or it changed while being read.
-template <int NT>
-__device__ bool adopt_best(SharedBest* g, const uint32_t* tours, const NearTour& T,
-                           unsigned long long best_len, NearShared<NT>& S) {
+template <int NT, typename SH>
+__device__ bool adopt_best(SharedBest* g, const uint32_t* tours, const CtaTour& T,
+                           unsigned long long best_len, SH& S) {
     if (threadIdx.x == 0) {
         const unsigned int q = ld_acquire_u32(&g->seq);
         const unsigned long long gl = *(volatile unsigned long long*)&g->best_len;
@@ -528,9 +528,9 @@ template <int NT>
 __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
     batch_kernel(BatchArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ NearShared<NT> S;
+    __shared__ NearShared<NT, 1, uint16_t> S;
     uint32_t parity = 0;
-    near_init<NT>(S);
+    S.init();
 
     for (;;) {
         if (threadIdx.x == 0) S.idx = atomicAdd(A.queue, 1u);
@@ -543,7 +543,8 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
         const uint32_t n = I.n;
         const float2* xy = A.coords + I.off;
         uint32_t* rio = A.routes + I.off;
-        NearTour T = near_carve(smem_raw, n);
+        CtaTour T = near_carve(smem_raw, n);
+        NearSeed seed;
 
         // load (or build) the start tour; rio holds the best tour from here on
         if (A.start == kStartNN) {  // the list area holds the builder's two arrays
@@ -570,7 +571,7 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
             // descent
             unsigned long long dm = 0;
             for (;;) {
-                const unsigned long long key = near_sweep<NT>(T, S, parity);
+                const unsigned long long key = near_sweep<NT, false>(T, S, seed, parity);
                 parity ^= 1u;
                 ++sweeps;
                 if (key == kNoMove) break;

@@ -54,9 +54,11 @@ struct logo_ctx {
     uint32_t* d_workctl = nullptr;
     uint32_t* d_pos = nullptr;    // boxed sweep: tour position of every city
     uint32_t* d_nbr = nullptr;    // boxed sweep: kSeedNeighbours nearest cities per city
-    CoopSync* d_coop = nullptr;   // barrier and best-key slots of the cooperative descent
-    int coop_grid = 0;            // CTAs of the cooperative descent (0: unavailable)
-    int coop_ils_grid = 0;        // CTAs of the cooperative ILS launch (0: unavailable)
+    CoopSync* d_coop = nullptr;   // barrier and best-key slots of the cooperative neighbour phase
+    NearIndex near{};             // neighbour lists and search grid (near_tour.cuh)
+    uint32_t* d_near = nullptr;   // its arrays
+    int solo_ctas = 0;            // CTAs of the one-cluster descent (0: unavailable)
+    int solo_ils_ctas = 0;        // the same for a whole ILS call
     int descent_mode = LOGO_DESCENT_AUTO;
     uint2* d_tiles = nullptr;
     uint32_t ntiles = 0;
@@ -165,6 +167,21 @@ SweepLaunch sweep_args(const logo_ctx* c) {
     L.pos = c->d_pos;
     L.nbr = c->d_nbr;
     return L;
+}
+
+SoloArgs solo_args(const logo_ctx* c) {
+    SoloArgs A{};
+    A.Q0 = c->d_Q[0];
+    A.Q1 = c->d_Q[1];
+    A.R0 = c->d_route[0];
+    A.R1 = c->d_route[1];
+    A.n = c->n;
+    A.st = c->d_st;
+    A.xy = c->d_xy;
+    A.near = c->near;
+    A.Qbest = c->d_Qbest;
+    A.route_best = c->d_route_best;
+    return A;
 }
 
 uint64_t pairs_of(uint32_t n) { return n < 4 ? 0 : (uint64_t)(n - 2) * (n - 3) / 2; }
@@ -590,8 +607,8 @@ std::mutex& coop_lock(int device) {
     return locks[(unsigned)device % 64];
 }
 
-bool use_coop(const logo_ctx* c) {
-    return c->coop_grid > 0 && c->descent_mode != LOGO_DESCENT_GRAPH &&
+bool use_solo(const logo_ctx* c) {
+    return c->solo_ctas > 0 && c->descent_mode != LOGO_DESCENT_GRAPH &&
            c->search == LOGO_SEARCH_EXHAUSTIVE;
 }
 
@@ -617,33 +634,19 @@ logo_status run_descent(logo_ctx* c, uint64_t max_moves, uint64_t* moves_out,
         moves0 = c->h_st->moves;
         sweeps0 = c->h_st->sweeps;
     }
-    if (use_coop(c)) {
-        // one cooperative launch runs the whole descent
-        CK(c, cudaMemsetAsync(c->d_coop, 0xFF, sizeof(CoopSync), c->stream));
-        CK(c, cudaMemsetAsync(c->d_coop, 0, 2 * sizeof(unsigned int), c->stream));
-        CoopArgs A;
-        A.Q0 = c->d_Q[0];
-        A.Q1 = c->d_Q[1];
-        A.R0 = c->d_route[0];
-        A.R1 = c->d_route[1];
-        A.n = c->n;
-        A.margin = c->margin;
-        A.st = c->d_st;
-        A.cs = c->d_coop;
+    if (use_solo(c)) {
+        // one cluster runs the whole descent
+        CK(c, launch_solo(solo_args(c), false, c->solo_ctas, c->stream));
         logo_status s;
-        {
-            std::lock_guard<std::mutex> lk(coop_lock(c->device));
-            CK(c, launch_coop_descent(A, c->coop_grid, c->stream));
-            if (route_out) {  // the launch runs the whole descent
-                s = enqueue_route_out(c, route_out, false);
-                if (s != LOGO_OK) return s;
-                if (route_stored) *route_stored = true;
-            }
-            s = read_state(c);
+        if (route_out) {  // the launch runs the whole descent
+            s = enqueue_route_out(c, route_out, false);
+            if (s != LOGO_OK) return s;
+            if (route_stored) *route_stored = true;
         }
+        s = read_state(c);
         if (s != LOGO_OK) return s;
         if (!c->h_st->converged && !c->h_st->status)
-            return fail(c, LOGO_ERR_DEVICE_FAULT, "cooperative descent did not finish");
+            return fail(c, LOGO_ERR_DEVICE_FAULT, "the descent did not finish");
     } else if (c->search != LOGO_SEARCH_EXHAUSTIVE) {
         // neighbour sweeps until no candidate improves (one cooperative
         // launch where available), then full sweeps
@@ -780,6 +783,7 @@ void destroy(logo_ctx* c) {
     cudaFree(c->d_start);
     if (c->nbr_chunk_exec) cudaGraphExecDestroy(c->nbr_chunk_exec);
     cudaFree(c->d_coop);
+    cudaFree(c->d_near);
     if (c->h_st) cudaFreeHost(c->h_st);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -913,14 +917,19 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     CKC(cudaMalloc(&c->d_rbox, sizeof(float4) * sweep_row_windows(n)));
     CKC(cudaMalloc(&c->d_rmax, sizeof(float) * sweep_row_windows(n)));
     CKC(cudaMalloc(&c->d_workctl, 3 * sizeof(uint32_t)));
-    c->coop_grid = coop_grid(n, device);
-    c->coop_ils_grid = c->coop_grid > 0 ? coop_ils_grid(n, device) : 0;
-    if (c->coop_grid > 0) CKC(cudaMalloc(&c->d_coop, sizeof(CoopSync)));
+    c->solo_ctas = solo_ctas(n, false);
+    c->solo_ils_ctas = c->solo_ctas > 0 ? solo_ctas(n, true) : 0;
     std::memset(c->h_st, 0, sizeof(DevState));
     c->h_st->best_key = kNoMove;
     c->h_st->converged = 1;
     CKC(cudaMemcpy(c->d_st, c->h_st, sizeof(DevState), cudaMemcpyHostToDevice));
     CKC(cudaMemcpy(c->d_xy, coords, sizeof(float2) * n, cudaMemcpyHostToDevice));
+    if (c->solo_ctas > 0) {
+        CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n)));
+        near_index_carve(c->near, c->d_near, n);
+        c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
+        CKC(launch_near_index(c->near, c->d_xy, n, c->stream));
+    }
 #undef CKC
     s = rebuild(c);
     if (s != LOGO_OK) return bail(s);
@@ -944,8 +953,8 @@ logo_status logo_ctx_get_info(const logo_ctx* c, logo_ctx_info* info) {
     info->filter_margin = c->margin;
     info->graph_steps = c->chunk_steps;
     info->variant = c->variant;
-    info->descent_mode = use_coop(c) ? LOGO_DESCENT_COOPERATIVE : LOGO_DESCENT_GRAPH;
-    info->cooperative_ctas = c->coop_grid;
+    info->descent_mode = use_solo(c) ? LOGO_DESCENT_COOPERATIVE : LOGO_DESCENT_GRAPH;
+    info->cooperative_ctas = c->solo_ctas;
     info->host_waits = c->host_waits;
     info->route_io = route_direct(c) ? LOGO_ROUTE_IO_DIRECT : LOGO_ROUTE_IO_COPY;
     info->search = c->search;
@@ -1017,7 +1026,7 @@ logo_status logo_ctx_set_descent_mode(logo_ctx* c, int mode) {
     if (mode != LOGO_DESCENT_AUTO && mode != LOGO_DESCENT_GRAPH &&
         mode != LOGO_DESCENT_COOPERATIVE)
         return fail(c, LOGO_ERR_INVALID_ARG, "unknown descent mode");
-    if (mode == LOGO_DESCENT_COOPERATIVE && c->coop_grid <= 0)
+    if (mode == LOGO_DESCENT_COOPERATIVE && c->solo_ctas <= 0)
         return fail(c, LOGO_ERR_INVALID_ARG,
                     "cooperative descent unavailable (n above 6,144 or device without it)");
     c->descent_mode = mode;
@@ -1297,8 +1306,8 @@ logo_status logo_ils(logo_ctx* c, uint32_t* route, uint32_t kicks, uint64_t seed
     if (kick_kind != LOGO_KICK_SEGMENT && kick_kind != LOGO_KICK_DOUBLE_BRIDGE)
         return fail(c, LOGO_ERR_INVALID_ARG, "unknown kick kind");
     CK(c, cudaSetDevice(c->device));
-    const bool coop = use_coop(c) && c->coop_ils_grid > 0;
-    if (!coop) {
+    const bool solo = use_solo(c) && c->solo_ils_ctas > 0;
+    if (!solo) {
         logo_status sb = build_ils_graph(c);  // once per context and tile shape
         if (sb != LOGO_OK) return sb;
     }
@@ -1322,26 +1331,12 @@ logo_status logo_ils(logo_ctx* c, uint32_t* route, uint32_t kicks, uint64_t seed
     CK(c, launch_save_best(bufs(c), c->stream));  // best = start, start_length recorded
     const uint64_t kmax = 64ull * c->n * c->n + 1024;
     CK(c, launch_reset_descent(bufs(c), kmax, c->stream));
-    if (coop) {
-        // one cooperative launch runs every descent, length, accept and kick
-        CK(c, cudaMemsetAsync(c->d_coop, 0xFF, sizeof(CoopSync), c->stream));
-        CK(c, cudaMemsetAsync(c->d_coop, 0, 2 * sizeof(unsigned int), c->stream));
-        CoopArgs A;
-        A.Q0 = c->d_Q[0];
-        A.Q1 = c->d_Q[1];
-        A.R0 = c->d_route[0];
-        A.R1 = c->d_route[1];
-        A.n = c->n;
-        A.margin = c->margin;
-        A.st = c->d_st;
-        A.cs = c->d_coop;
-        A.xy = c->d_xy;
-        A.Qbest = c->d_Qbest;
-        A.route_best = c->d_route_best;
+    if (solo) {
+        // one cluster runs every descent, length, accept and kick
+        SoloArgs A = solo_args(c);
         A.kicks = kicks;
         A.kick_kind = kick_kind;
-        std::lock_guard<std::mutex> lk(coop_lock(c->device));
-        CK(c, launch_coop_ils(A, c->coop_ils_grid, c->stream));
+        CK(c, launch_solo(A, true, c->solo_ils_ctas, c->stream));
         s = read_state(c);
     } else {
         // one graph: descent and kick loops are WHILE nodes on device conditions

@@ -192,13 +192,13 @@ __device__ __forceinline__ void chain_release() {
 }
 
 // ---- warp / block reductions ----------------------------------------------
+// (two 32-bit warp reductions: the upper halves, then the lower halves of
+// those that tie)
 __device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        uint64_t w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-    }
-    return v;
+    const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(v >> 32));
+    const uint32_t lo =
+        __reduce_min_sync(0xffffffffu, (uint32_t)(v >> 32) == hi ? (uint32_t)v : 0xffffffffu);
+    return (uint64_t)hi << 32 | lo;
 }
 __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
 #pragma unroll

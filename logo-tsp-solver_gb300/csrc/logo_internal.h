@@ -6,6 +6,7 @@
 
 #include "../../include/logo_gpu.h"
 #include "logo_device.cuh"
+#include "near_grid.h"
 
 namespace logo {
 
@@ -137,41 +138,58 @@ struct TourBufs {
     // kept current by every kernel that moves the tour
     uint32_t* pos;
 };
-// Cooperative persistent descent (coop.cu) for tours up to kCoopMaxN cities:
-// one launch runs the descent to a local optimum or st->max_moves.
-constexpr uint32_t kCoopMaxN = 6144;
+// Neighbours per city in a context's lists: few walks run off 40 (counted on
+// the CPU, slots whose list is too short per sweep of the descent with 16 and
+// with 32: n = 1,000 from the NN tour 12.5 and 3.5, n = 6,000 clustered 105
+// and 34, after a kick at n = 1,500 4.8 and 1.4).
+constexpr uint32_t kCtxNear = 40;
+// Neighbour lists and search grid of a context's cities (near_tour.cuh),
+// built on the device once per context.
+struct NearIndex {
+    uint32_t* nbr;
+    uint32_t* cell;
+    uint32_t* cellid;
+    NearGrid g;
+};
+// 32-bit words behind nbr, cell and cellid.
+size_t near_index_words(uint32_t n);
+void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);
+cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s);
+
+// One cluster runs a whole descent, or a whole ILS call, of a tour of 8 to
+// kSoloMaxN cities (solo.cu).
+constexpr uint32_t kSoloMaxN = 6144;
+struct SoloArgs {
+    OrderedCity* Q0;
+    OrderedCity* Q1;
+    uint32_t* R0;
+    uint32_t* R1;
+    uint32_t n;
+    DevState* st;
+    const float2* xy;  // coordinates by city id
+    NearIndex near;
+    // ILS only: the best tour (also the start: route_best/Qbest and
+    // st->best_length are set before the launch), the kick count and kind
+    OrderedCity* Qbest;
+    uint32_t* route_best;
+    uint32_t kicks;
+    int kick_kind;
+};
+// CTAs of the cluster for this n on the current device (0: not available).
+uint32_t solo_wanted_ctas(uint32_t n);
+int solo_ctas(uint32_t n, bool ils);
+// Without ils: a descent to a local optimum or st->max_moves.  With ils:
+// descent, length, accept/revert and kicks for A.kicks kicks
+// (ILSGlobalSolverSequential::optimize with a kick count).
+cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s);
+
+// State of a cooperative launch (coop.cu).
 struct CoopSync {
     unsigned int count;            // CTAs arrived at the current barrier
     unsigned int gen;              // barrier generation
     unsigned long long slot[3];    // best key of move m in slot m % 3
     unsigned long long or_slot[3][5];  // neighbour phase: Or-opt keys per variant
 };
-struct CoopArgs {
-    OrderedCity* Q0;
-    OrderedCity* Q1;
-    uint32_t* R0;
-    uint32_t* R1;
-    uint32_t n;
-    float margin;
-    DevState* st;
-    CoopSync* cs;  // count = gen = 0 and every slot = kNoMove before the launch
-    // ILS launch only: coordinates by city id, the best tour (also the start:
-    // route_best/Qbest and st->best_length are set before the launch) and the
-    // kick count and kind
-    const float2* xy;
-    OrderedCity* Qbest;
-    uint32_t* route_best;
-    uint32_t kicks;
-    int kick_kind;
-};
-// CTAs for a cooperative launch at this n on `device` (0: not available);
-// coop_ils_grid for the launch that runs a whole ILS call.
-int coop_grid(uint32_t n, int device);
-int coop_ils_grid(uint32_t n, int device);
-cudaError_t launch_coop_descent(const CoopArgs& A, int grid, cudaStream_t s);
-// One cooperative launch runs descent, length, accept/revert and kicks for
-// A.kicks kicks (ILSGlobalSolverSequential::optimize with a kick count).
-cudaError_t launch_coop_ils(const CoopArgs& A, int grid, cudaStream_t s);
 // One CTA waits at the cooperative grid barrier sized for two (test hook).
 cudaError_t launch_barrier_probe(CoopSync* cs, DevState* st, cudaStream_t s);
 

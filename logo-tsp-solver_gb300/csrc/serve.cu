@@ -35,9 +35,9 @@ template <int NT>
 __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
     serve_round_kernel(ServeArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ NearShared<NT> S;
+    __shared__ NearShared<NT, 1, uint16_t> S;
     uint32_t parity = 0;
-    near_init<NT>(S);
+    S.init();
 
     for (;;) {
         if (threadIdx.x == 0) S.idx = atomicAdd(A.queue, 1u);
@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
         const float2* xy = A.coords + st.off;
         uint32_t* rio = A.route + st.off;
         uint32_t* bio = A.best + st.off;
-        NearTour T = near_carve(smem_raw, n);
+        CtaTour T = near_carve(smem_raw, n);
+        NearSeed seed;
 
         // load the resident tour into shared memory (the best one stays in the arena)
         for (uint32_t k = threadIdx.x; k < n; k += NT) {
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
         uint64_t rng = st.rng;
         while (st.phase != kServeDone && spent < A.budget_pairs) {
             if (st.phase == kServeDescent) {
-                const unsigned long long key = near_sweep<NT>(T, S, parity);
+                const unsigned long long key = near_sweep<NT, false>(T, S, seed, parity);
                 parity ^= 1u;
                 ++st.sweeps;
                 spent += kServePairsPerCity * n;

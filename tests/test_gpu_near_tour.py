@@ -58,3 +58,37 @@ def test_points_of_every_shape(lg, inst, oracle_mod, kind):
 def test_largest_instance(lg, inst, oracle_mod):
     xy = inst.clustered(4096, 2, clusters=20, sigma_frac=0.03)
     check(lg, oracle_mod, [xy], [lg.nn_tour(xy)], [9], 1, 1)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "line", "heaps", "clumps", "offset", "lattice"])
+@pytest.mark.parametrize("n", [8, 9, 40, 41, 42, 64, 65, 130, 1025])
+def test_one_cluster_descent_and_ils(lg, inst, oracle_mod, n, kind):
+    """A context's small instance solved by one cluster: from one CTA to
+    sixteen, with lists that hold every other city and lists that do not."""
+    xy = points(inst, kind, n, 40 + n)
+    r = inst.random_tour(n, n)
+    with lg.Solver(xy) as s:
+        assert s.info()["descent_mode"] == lg.DESCENT_COOPERATIVE
+        got, st = s.optimize(r)
+        want, moves, _ = oracle_mod.descend(xy, r)
+        assert np.array_equal(got, want) and st["moves"] == moves
+        got, st = s.ils(want, 3, 7, n % 2)
+        want, ost = oracle_mod.ils(xy, want, 3, 7, kind=n % 2)
+        assert np.array_equal(got, want) and st["final_length"] == ost["best_length"]
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 4097])
+def test_one_cluster_and_graph_agree(lg, inst, n):
+    """Where the cluster's threads change, and above the sizes the oracle
+    walks quickly: the graph-driven descent has the same moves."""
+    xy = inst.clustered(n, n, clusters=20, sigma_frac=0.03)
+    r = lg.nn_tour(xy)
+    res = []
+    for mode in (lg.DESCENT_GRAPH, lg.DESCENT_COOPERATIVE):
+        with lg.Solver(xy) as s:
+            s.set_descent_mode(mode)
+            t, tr, st = s.optimize_trace(r)
+            u, su = s.ils(t, 3, 5, 1)
+        res.append((t, tr, st["sweeps"], u, su["final_length"], su["moves"], su["sweeps"]))
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
