@@ -53,12 +53,14 @@ struct logo_ctx {
     uint4* d_work = nullptr;      // boxed sweep: tiles that pass the window test
     uint32_t* d_workctl = nullptr;
     uint32_t* d_pos = nullptr;    // boxed sweep: tour position of every city
-    uint32_t* d_nbr = nullptr;    // boxed sweep: kSeedNeighbours nearest cities per city
     CoopSync* d_coop = nullptr;   // barrier and best-key slots of the cooperative neighbour phase
     NearIndex near{};             // neighbour lists and search grid (near_tour.cuh)
     uint32_t* d_near = nullptr;   // its arrays
     int solo_ctas = 0;            // CTAs of the one-cluster descent (0: unavailable)
     int solo_ils_ctas = 0;        // the same for a whole ILS call
+    int grid_ctas = 0;            // CTAs of the grid-wide descent of larger tours (0: unavailable)
+    GridSync* d_grid = nullptr;
+    bool own_kernel = false;      // the caller chose a sweep kernel: descents run that one
     int descent_mode = LOGO_DESCENT_AUTO;
     uint2* d_tiles = nullptr;
     uint32_t ntiles = 0;
@@ -165,7 +167,7 @@ SweepLaunch sweep_args(const logo_ctx* c) {
     L.R0 = c->d_route[0];
     L.R1 = c->d_route[1];
     L.pos = c->d_pos;
-    L.nbr = c->d_nbr;
+    L.nbr = c->near.nbr;
     return L;
 }
 
@@ -181,6 +183,14 @@ SoloArgs solo_args(const logo_ctx* c) {
     A.near = c->near;
     A.Qbest = c->d_Qbest;
     A.route_best = c->d_route_best;
+    return A;
+}
+
+GridArgs grid_args(const logo_ctx* c) {
+    GridArgs A{};
+    A.solo = solo_args(c);
+    A.pos = c->d_pos;
+    A.gs = c->d_grid;
     return A;
 }
 
@@ -281,20 +291,11 @@ logo_status rebuild(logo_ctx* c) {
         cudaFree(c->d_work);
         c->d_work = nullptr;
     }
-    if (c->variant == LOGO_SWEEP_BOXED && !c->d_nbr) {
-        // near neighbours of every city, once per context: the boxed sweep's
-        // seed pass evaluates their pairs first (host grid search)
-        std::vector<logo_xy> h(c->n);
-        CK(c, cudaMemcpy(h.data(), c->d_xy, sizeof(logo_xy) * c->n, cudaMemcpyDeviceToHost));
-        std::vector<uint32_t> nb((size_t)c->n * kSeedNeighbours);
-        knn_grid(h.data(), c->n, kSeedNeighbours, nb.data());
-        CK(c, cudaMalloc(&c->d_pos, sizeof(uint32_t) * c->n));
+    if (c->variant == LOGO_SWEEP_BOXED && !c->d_pos) {
         // positions are written by every kernel that moves the tour; until a
         // route is uploaded they only need to be in range
+        CK(c, cudaMalloc(&c->d_pos, sizeof(uint32_t) * c->n));
         CK(c, cudaMemset(c->d_pos, 0, sizeof(uint32_t) * c->n));
-        CK(c, cudaMalloc(&c->d_nbr, sizeof(uint32_t) * nb.size()));
-        CK(c, cudaMemcpy(c->d_nbr, nb.data(), sizeof(uint32_t) * nb.size(),
-                         cudaMemcpyHostToDevice));
     }
     std::vector<uint2> tiles = make_tiles(c->n, c->R, c->NW, c->cb);
     c->ntiles = (uint32_t)tiles.size();
@@ -612,6 +613,13 @@ bool use_solo(const logo_ctx* c) {
            c->search == LOGO_SEARCH_EXHAUSTIVE;
 }
 
+// Larger tours: the grid-wide launch, unless the caller asked for graphs or
+// chose the sweep kernel that descents are to run.
+bool use_grid(const logo_ctx* c) {
+    return c->grid_ctas > 0 && c->descent_mode == LOGO_DESCENT_AUTO && !c->own_kernel &&
+           c->search == LOGO_SEARCH_EXHAUSTIVE;
+}
+
 // reset_enqueued: the reset was folded into the route load just before.
 // route_out (direct route mode only): the caller's buffer, written on the
 // device before the final state read when the descent is known to end there
@@ -634,11 +642,17 @@ logo_status run_descent(logo_ctx* c, uint64_t max_moves, uint64_t* moves_out,
         moves0 = c->h_st->moves;
         sweeps0 = c->h_st->sweeps;
     }
-    if (use_solo(c)) {
-        // one cluster runs the whole descent
-        CK(c, launch_solo(solo_args(c), false, c->solo_ctas, c->stream));
+    if (use_solo(c) || use_grid(c)) {
+        // one launch runs the whole descent: a cluster, or the whole device
+        std::unique_lock<std::mutex> lk;
+        if (use_solo(c)) {
+            CK(c, launch_solo(solo_args(c), false, c->solo_ctas, c->stream));
+        } else {
+            lk = std::unique_lock<std::mutex>(coop_lock(c->device));
+            CK(c, launch_near_grid(grid_args(c), false, c->grid_ctas, c->stream));
+        }
         logo_status s;
-        if (route_out) {  // the launch runs the whole descent
+        if (route_out) {
             s = enqueue_route_out(c, route_out, false);
             if (s != LOGO_OK) return s;
             if (route_stored) *route_stored = true;
@@ -778,12 +792,12 @@ void destroy(logo_ctx* c) {
     cudaFree(c->d_work);
     cudaFree(c->d_workctl);
     cudaFree(c->d_pos);
-    cudaFree(c->d_nbr);
     cudaFree(c->d_nbr_search);
     cudaFree(c->d_start);
     if (c->nbr_chunk_exec) cudaGraphExecDestroy(c->nbr_chunk_exec);
     cudaFree(c->d_coop);
     cudaFree(c->d_near);
+    cudaFree(c->d_grid);
     if (c->h_st) cudaFreeHost(c->h_st);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -924,12 +938,16 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     c->h_st->converged = 1;
     CKC(cudaMemcpy(c->d_st, c->h_st, sizeof(DevState), cudaMemcpyHostToDevice));
     CKC(cudaMemcpy(c->d_xy, coords, sizeof(float2) * n, cudaMemcpyHostToDevice));
-    if (c->solo_ctas > 0) {
-        CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n)));
-        near_index_carve(c->near, c->d_near, n);
-        c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
-        CKC(launch_near_index(c->near, c->d_xy, n, c->stream));
+    c->grid_ctas = near_grid_ctas(n, device);
+    if (c->grid_ctas > 0) {
+        CKC(cudaMalloc(&c->d_grid, sizeof(GridSync)));
+        CKC(cudaMalloc(&c->d_pos, sizeof(uint32_t) * n));
+        CKC(cudaMemset(c->d_pos, 0, sizeof(uint32_t) * n));
     }
+    CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n)));
+    near_index_carve(c->near, c->d_near, n);
+    c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
+    CKC(launch_near_index(c->near, c->d_xy, n, c->stream));
 #undef CKC
     s = rebuild(c);
     if (s != LOGO_OK) return bail(s);
@@ -1044,6 +1062,7 @@ logo_status logo_ctx_set_shape(logo_ctx* c, int R, int NW, uint32_t cb) {
     c->R = R;
     c->NW = NW;
     c->cb = cb;
+    c->own_kernel = true;
     return rebuild(c);
 }
 
@@ -1062,6 +1081,7 @@ logo_status logo_ctx_set_kernel(logo_ctx* c, int variant, int R, int NW, uint32_
     c->R = R;
     c->NW = NW;
     c->cb = cb;
+    c->own_kernel = true;
     return rebuild(c);
 }
 
@@ -1306,8 +1326,8 @@ logo_status logo_ils(logo_ctx* c, uint32_t* route, uint32_t kicks, uint64_t seed
     if (kick_kind != LOGO_KICK_SEGMENT && kick_kind != LOGO_KICK_DOUBLE_BRIDGE)
         return fail(c, LOGO_ERR_INVALID_ARG, "unknown kick kind");
     CK(c, cudaSetDevice(c->device));
-    const bool solo = use_solo(c) && c->solo_ils_ctas > 0;
-    if (!solo) {
+    const bool solo = use_solo(c) && c->solo_ils_ctas > 0, grid = use_grid(c);
+    if (!solo && !grid) {
         logo_status sb = build_ils_graph(c);  // once per context and tile shape
         if (sb != LOGO_OK) return sb;
     }
@@ -1337,6 +1357,13 @@ logo_status logo_ils(logo_ctx* c, uint32_t* route, uint32_t kicks, uint64_t seed
         A.kicks = kicks;
         A.kick_kind = kick_kind;
         CK(c, launch_solo(A, true, c->solo_ils_ctas, c->stream));
+        s = read_state(c);
+    } else if (grid) {
+        GridArgs A = grid_args(c);
+        A.solo.kicks = kicks;
+        A.solo.kick_kind = kick_kind;
+        std::lock_guard<std::mutex> lk(coop_lock(c->device));
+        CK(c, launch_near_grid(A, true, c->grid_ctas, c->stream));
         s = read_state(c);
     } else {
         // one graph: descent and kick loops are WHILE nodes on device conditions

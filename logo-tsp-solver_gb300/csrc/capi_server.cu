@@ -102,9 +102,13 @@ private:
 
 constexpr uint64_t kSmallBytesPerCity = sizeof(float2) + 2 * sizeof(uint32_t);
 // device bytes per city of the single-instance path (coordinates, two tour
-// buffers of ordered cities and routes, best tour, and the boxed sweep's city
-// positions and near-neighbour lists)
-constexpr uint64_t kLargeBytesPerCity = 8 + 2 * 16 + 2 * 4 + 16 + 4 + 4 * (1 + kSeedNeighbours);
+// buffers of ordered cities and routes, best tour, the boxed sweep's city
+// positions and near-neighbour lists, and the neighbour lists and cells of the
+// descents); a request that the budget holds but for those last is run alone
+constexpr uint64_t kLargeLeastBytesPerCity =
+    8 + 2 * 16 + 2 * 4 + 16 + 4 + 4 * (1 + kSeedNeighbours);
+constexpr uint64_t kLargeBytesPerCity =
+    kLargeLeastBytesPerCity + 8 * kCtxNear - 4 * kSeedNeighbours + 4 + 2;
 
 thread_local std::string g_server_err;
 
@@ -227,7 +231,9 @@ void admit(logo_server* s) {
         Req& r = s->reqs[*it];
         bool ok = false;
         if (r.large) {
-            const uint64_t mem = kLargeBytesPerCity * r.n;
+            uint64_t mem = kLargeBytesPerCity * r.n;
+            if (mem > s->opts.mem_budget)
+                mem = std::max(kLargeLeastBytesPerCity * r.n, s->opts.mem_budget);
             if (s->running_large < s->opts.max_large && s->mem_in_use + mem <= s->opts.mem_budget) {
                 r.mem = mem;
                 s->mem_in_use += mem;

@@ -61,12 +61,13 @@ struct SweepLaunch {
     uint4* work;         // ntiles entries
     uint32_t* workctl;   // tiles listed from the start, claimed, listed from the end
     // boxed variant: the tour's city ids (both buffers), the tour position of
-    // every city (written by the window pass) and kSeedNeighbours nearest
-    // neighbours per city, whose pairs seed the sweep's best delta
+    // every city (kept by every kernel that moves the tour) and the context's
+    // neighbour lists (NearIndex), the pairs of whose first kSeedNeighbours
+    // entries seed the sweep's best delta
     const uint32_t* R0;
     const uint32_t* R1;
     uint32_t* pos;
-    const uint32_t* nbr;
+    const uint2* nbr;
 };
 constexpr uint32_t kSeedNeighbours = 5;
 // k nearest other cities of every city, out[v * k + j] (construct.cpp).
@@ -146,14 +147,14 @@ constexpr uint32_t kCtxNear = 40;
 // Neighbour lists and search grid of a context's cities (near_tour.cuh),
 // built on the device once per context.
 struct NearIndex {
-    uint32_t* nbr;
+    uint2* nbr;  // kCtxNear entries per city: city, squared distance (near_tour.cuh)
     uint32_t* cell;
     uint32_t* cellid;
     NearGrid g;
 };
 // 32-bit words behind nbr, cell and cellid.
 size_t near_index_words(uint32_t n);
-void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);
+void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);  // words 8-byte aligned
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s);
 
 // One cluster runs a whole descent, or a whole ILS call, of a tour of 8 to
@@ -182,6 +183,23 @@ int solo_ctas(uint32_t n, bool ils);
 // descent, length, accept/revert and kicks for A.kicks kicks
 // (ILSGlobalSolverSequential::optimize with a kick count).
 cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s);
+
+// A descent or an ILS call of a larger tour as one cooperative launch over the
+// whole device (grid_tour.cu): one CTA per SM.
+constexpr uint32_t kGridMaxCtas = 256;
+struct GridSync {
+    unsigned long long arrived;    // barrier arrivals so far
+    unsigned long long length[2];  // tour length of the descent in hand, by its parity
+    unsigned long long keys[2][kGridMaxCtas];  // best key per CTA, by the sweep's parity
+};
+struct GridArgs {
+    SoloArgs solo;
+    uint32_t* pos;  // slot of every city; positions again when the launch ends
+    GridSync* gs;
+};
+// CTAs of the launch (0: n is not above kSoloMaxN, or not available).
+int near_grid_ctas(uint32_t n, int device);
+cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t s);
 
 // State of a cooperative launch (coop.cu).
 struct CoopSync {

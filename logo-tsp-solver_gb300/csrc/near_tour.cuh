@@ -79,6 +79,32 @@ __host__ __device__ constexpr NearLayout near_layout(uint32_t n) {
     return l;
 }
 
+// The squared distance whose rounded root the per-edge distance is
+// (exact_dist in logo_device.cuh).
+__device__ __forceinline__ float near_sq(float2 a, float2 b) {
+    const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y);
+    return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+}
+// Lengths are whole numbers below 2^21 kept in binary32: sums of four are exact,
+// and nothing on the way needs a conversion.
+__device__ __forceinline__ float near_len(float s) {
+    return truncf(__fadd_rn(__fsqrt_rn(s), 0.5f));
+}
+__device__ __forceinline__ float near_dist(float2 a, float2 b) { return near_len(near_sq(a, b)); }
+
+// An entry of a neighbour list.  In global memory it carries its squared distance,
+// so that an entry out of reach costs one dependent read, not three; in shared
+// memory, where reads are quick and room is short, it does not.
+template <typename IX>
+struct NearEntry {
+    IX id;
+};
+template <>
+struct __align__(8) NearEntry<uint32_t> {
+    uint32_t id;
+    float s;
+};
+
 // IX: what a city or slot number is stored as (uint16_t where all arrays are in
 // one CTA's shared memory, else uint32_t); KN: neighbours per list.
 template <typename IX, uint32_t KN>
@@ -95,7 +121,7 @@ struct NearTour {
     float* E;       // by slot: the length of the edge between slots j - 1 and j
     IX* id;     // city in slot j
     IX* pos;    // slot of city v
-    IX* nbr;
+    NearEntry<IX>* nbr;
     IX* cell;    // first entry of every cell in cellid (row major), and the end
     IX* cellid;  // cities by cell
     NearGrid g;
@@ -110,6 +136,14 @@ struct NearTour {
         if (!rev) return j >= o ? j - o : j + n - o;
         const uint32_t t = o + 1;  // (o + 1 - j) mod n
         return t >= j ? (t - j == n ? 0u : t - j) : t + n - j;
+    }
+    // squared distance of the last entry of the list of the city in slot j
+    __device__ __forceinline__ float last_sq(uint32_t j) const {
+        const NearEntry<IX> e = nbr[id[j] * KN + KN - 1];
+        if constexpr (sizeof(IX) == 4)
+            return e.s;
+        else
+            return near_sq(xy[j], xy[pos[e.id]]);
     }
     // where E holds the closing edge
     __device__ __forceinline__ uint32_t closing() const { return rev ? wrap(o + 1) : o; }
@@ -129,16 +163,26 @@ struct NearShared {
     uint32_t scan[NT / 32];
     // by the sweep's parity: best delta met, entries of far and wide (more may
     // have been offered than fit)
-    int bound[2];
+    int bound[2], far_bound[2];  // (of its lists, and of its discs)
     uint32_t fars[2], big[2];
     IX far[kNearFar];         // slots whose lists were too short
     IX wide[kNearWide];       // those of them whose discs are large
-    IX scratch[NT / 32][32];  // each warp's slots in hand
+    // each warp's slots in hand: slot, its city, its longer edge
+    struct Slots {
+        IX j[32], id[32], open[32];
+        float m[32];
+    } slots[NT / 32];
+    // each warp's pairs of slots that are in reach of one another: slot, slot of
+    // the other city (uint32_t: the other city), squared distance
+    struct Reach {
+        IX j[64], p[64];
+        float s[64];
+    } reach[NT / 32];
     uint32_t idx;
     unsigned int flag, seq;
 
     __device__ __forceinline__ void reset(uint32_t parity) {
-        bound[parity] = -1;
+        bound[parity] = far_bound[parity] = -1;
         fars[parity] = big[parity] = 0;
     }
     // once per kernel; a barrier must follow before the first sweep
@@ -166,24 +210,11 @@ __device__ __forceinline__ CtaTour near_carve(unsigned char* smem, uint32_t n) {
     T.E = reinterpret_cast<float*>(smem + l.e);
     T.id = reinterpret_cast<uint16_t*>(smem + l.id);
     T.pos = reinterpret_cast<uint16_t*>(smem + l.pos);
-    T.nbr = reinterpret_cast<uint16_t*>(smem + l.nbr);
+    T.nbr = reinterpret_cast<NearEntry<uint16_t>*>(smem + l.nbr);
     T.cell = reinterpret_cast<uint16_t*>(smem + l.cell);
     T.cellid = reinterpret_cast<uint16_t*>(smem + l.cellid);
     return T;
 }
-
-// The squared distance whose rounded root the per-edge distance is
-// (exact_dist in logo_device.cuh).
-__device__ __forceinline__ float near_sq(float2 a, float2 b) {
-    const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y);
-    return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-}
-// Lengths are whole numbers below 2^21 kept in binary32: sums of four are exact,
-// and nothing on the way needs a conversion.
-__device__ __forceinline__ float near_len(float s) {
-    return truncf(__fadd_rn(__fsqrt_rn(s), 0.5f));
-}
-__device__ __forceinline__ float near_dist(float2 a, float2 b) { return near_len(near_sq(a, b)); }
 
 // Cell column (or row) of a coordinate u counted from the box's corner:
 // monotone in u, clamped to the grid.  (Differences from the corner are below
@@ -200,7 +231,7 @@ __device__ __forceinline__ int near_cell(float u, float inv, int cells) {
 // nearer than r cells has been seen; a little less, for rounding).
 template <typename IX, uint32_t KN>
 __device__ void near_search(uint32_t v, const float2* __restrict__ gxy, const NearGrid& g,
-                            const IX* cell, const IX* cellid, IX* nbr) {
+                            const IX* cell, const IX* cellid, NearEntry<IX>* nbr) {
     const float2 p = gxy[v];
     const int cx = near_cell(p.x - g.x0, g.inv, g.gx), cy = near_cell(p.y - g.y0, g.inv, g.gy);
     float ds[KN];
@@ -249,7 +280,12 @@ __device__ void near_search(uint32_t v, const float2* __restrict__ gxy, const Ne
         }
     }
 #pragma unroll
-    for (uint32_t k = 0; k < KN; ++k) nbr[(size_t)v * KN + k] = (IX)vs[k];
+    for (uint32_t k = 0; k < KN; ++k) {
+        NearEntry<IX> e;
+        e.id = (IX)vs[k];
+        if constexpr (sizeof(IX) == 4) e.s = ds[k];
+        nbr[(size_t)v * KN + k] = e;
+    }
 }
 
 // Once per instance of a CTA: bounding box, counting sort of the cities into
@@ -364,14 +400,16 @@ __device__ __forceinline__ unsigned long long near_length(const TOUR& T, SH& S) 
     return s;
 }
 
-// Reverses the arc of len slots from slot u (len < n).  Slots and the inner
-// edges swap pairwise, the two outer edges get their new lengths from the
-// thread that holds the arc's ends.  A barrier must follow.
-template <int NT, typename TOUR>
-__device__ __forceinline__ void near_reverse(TOUR& T, uint32_t u, uint32_t len) {
+// Reverses the arc of len slots from slot u (len < n), by `threads` threads of
+// which this is number `tid`.  Slots and the inner edges swap pairwise, the two
+// outer edges get their new lengths from the thread that holds the arc's ends.
+// A barrier of all of them must follow.
+template <typename TOUR>
+__device__ __forceinline__ void near_reverse(TOUR& T, uint32_t u, uint32_t len, uint32_t tid,
+                                             uint32_t threads) {
     const uint32_t n = T.n;
     if (len == 0) return;
-    for (uint32_t t = threadIdx.x; t < (len + 1) / 2; t += NT) {
+    for (uint32_t t = tid; t < (len + 1) / 2; t += threads) {
         const uint32_t a = T.wrap(u + t), b = T.wrap(u + len - 1 - t);
         const float2 pa = T.xy[a], pb = T.xy[b];
         if (t == 0) {
@@ -386,7 +424,7 @@ __device__ __forceinline__ void near_reverse(TOUR& T, uint32_t u, uint32_t len) 
         T.pos[vb] = (typename TOUR::Index)a;
         T.pos[va] = (typename TOUR::Index)b;
     }
-    for (uint32_t t = threadIdx.x + 1; 2 * t < len; t += NT) {
+    for (uint32_t t = tid + 1; 2 * t < len; t += threads) {
         const uint32_t a = T.wrap(u + t), b = T.wrap(u + len - t);
         const float ea = T.E[a], eb = T.E[b];
         T.E[a] = eb;
@@ -395,42 +433,54 @@ __device__ __forceinline__ void near_reverse(TOUR& T, uint32_t u, uint32_t len) 
 }
 
 // Reverses positions [a, b) in place.
-template <int NT, typename TOUR>
-__device__ __forceinline__ void near_reverse_positions(TOUR& T, uint32_t a, uint32_t b) {
-    if (b <= a) return;
-    near_reverse<NT>(T, T.rev ? T.slot(b - 1) : T.slot(a), b - a);
+template <typename TOUR>
+__device__ __forceinline__ void near_reverse_positions(TOUR& T, uint32_t a, uint32_t b,
+                                                       uint32_t tid, uint32_t threads) {
+    if (b > a) near_reverse(T, T.rev ? T.slot(b - 1) : T.slot(a), b - a, tid, threads);
 }
 
-// new = old[p..q) ++ rev(old[0..p)) ++ rev(old[q..n)), p <= q < n.
-template <int NT, typename TOUR>
-__device__ __forceinline__ void near_move(TOUR& T, uint32_t p, uint32_t q) {
+// new = old[p..q) ++ rev(old[0..p)) ++ rev(old[q..n)), p <= q < n; a barrier of
+// all threads must follow.
+template <typename TOUR>
+__device__ __forceinline__ void near_move(TOUR& T, uint32_t p, uint32_t q, uint32_t tid,
+                                          uint32_t threads) {
     const uint32_t n = T.n, len = q - p;
     if (2 * len <= n) {
         // reversed arc [p, q), read the other way round from its far end
         const uint32_t first = T.slot(p), last = T.slot(q == 0 ? n - 1 : q - 1);
-        near_reverse<NT>(T, T.rev ? last : first, len);
+        near_reverse(T, T.rev ? last : first, len, tid, threads);
         T.o = last;
         T.rev = !T.rev;
     } else {
         // the complement: positions q .. n - 1, 0 .. p - 1
         const uint32_t o = T.slot(p);
-        near_reverse<NT>(T, T.rev ? T.slot(p == 0 ? n - 1 : p - 1) : T.slot(q), n - len);
+        near_reverse(T, T.rev ? T.slot(p == 0 ? n - 1 : p - 1) : T.slot(q), n - len, tid, threads);
         T.o = o;
     }
+}
+template <int NT, typename TOUR>
+__device__ __forceinline__ void near_move(TOUR& T, uint32_t p, uint32_t q) {
+    near_move(T, p, q, threadIdx.x, NT);
     __syncthreads();
 }
 
-// new = old[0,p1) old[p2,p3) old[p1,p2) old[p3,n).
+// new = old[0,p1) old[p2,p3) old[p1,p2) old[p3,n): three reversals in place, with
+// a barrier of all threads after each.
+template <typename TOUR, typename BAR>
+__device__ __forceinline__ void near_double_bridge(TOUR& T, uint32_t p1, uint32_t p2, uint32_t p3,
+                                                   uint32_t tid, uint32_t threads, BAR barrier) {
+    near_reverse_positions(T, p1, p3, tid, threads);
+    barrier();
+    const uint32_t m = p1 + (p3 - p2);
+    near_reverse_positions(T, p1, m, tid, threads);
+    barrier();
+    near_reverse_positions(T, m, p3, tid, threads);
+    barrier();
+}
 template <int NT, typename TOUR>
 __device__ __forceinline__ void near_double_bridge(TOUR& T, uint32_t p1, uint32_t p2,
                                                    uint32_t p3) {
-    near_reverse_positions<NT>(T, p1, p3);
-    __syncthreads();
-    const uint32_t m = p1 + (p3 - p2);
-    near_reverse_positions<NT>(T, p1, m);
-    __syncthreads();
-    near_reverse_positions<NT>(T, m, p3);
-    __syncthreads();
+    near_double_bridge(T, p1, p2, p3, threadIdx.x, NT, [] { __syncthreads(); });
 }
 
 // ---- the sweep --------------------------------------------------------------------
@@ -520,16 +570,17 @@ __device__ __forceinline__ bool near_meet(const TOUR& T, bool in, uint32_t j, ui
 }
 
 // A slot whose list was too short, looked at by the whole warp: the grid's
-// cells in the disc, of whose cities this warp takes part `part` of `parts`.  j
-// is the slot (the same in every lane).  A disc of more than `most` cities is
-// left alone, and the result is true.
+// cells in the disc that bound B gives, of whose cities this warp takes part
+// `part` of `parts` (B has to be the same in all of those warps: they number the
+// disc's cities alike).  j is the slot (the same in every lane).  A disc of more
+// than `most` cities is left alone, and the result is true.
 template <typename TOUR>
 __device__ __forceinline__ bool near_far(const TOUR& T, uint32_t j, uint32_t z,
-                                         uint32_t most, NearBest& nb, uint32_t part = 0,
-                                         uint32_t parts = 1) {
+                                         uint32_t most, float B, NearBest& nb,
+                                         uint32_t part = 0, uint32_t parts = 1) {
     const uint32_t lane = threadIdx.x & 31, jn = T.wrap(j + 1);
     const float ej = j == z ? kNoEdge : T.E[j], en = jn == z ? kNoEdge : T.E[jn];
-    const float V = fmaxf(ej, en) + near_half(nb.B);
+    const float V = fmaxf(ej, en) + near_half(B);
     if (V < 0.f) return false;
     const float2 p = T.xy[j];
     const float r = V + 2.f, lim = near_limit(V);
@@ -572,55 +623,110 @@ __device__ __forceinline__ bool near_far(const TOUR& T, uint32_t j, uint32_t z,
     return false;
 }
 
-// Entries FIRST .. FIRST + WIDTH - 1 of the lists of the slots from[0 .. count),
-// a lane per entry and 32 / WIDTH slots at a time (a long list keeps no other
-// slot waiting), SETS times that many in flight.  Writes the slots whose
-// entries were all in reach to out (which may be `from`) and returns their
-// number.
-template <uint32_t FIRST, uint32_t WIDTH, int SETS, typename TOUR>
-__device__ __forceinline__ uint32_t near_lists(const TOUR& T, const typename TOUR::Index* from,
-                                               uint32_t count, typename TOUR::Index* out,
-                                               uint32_t z, NearBest& nb) {
-    constexpr uint32_t SLOTS = 32 / WIDTH;
-    const uint32_t lane = threadIdx.x & 31, k = FIRST + lane % WIDTH;
-    uint32_t open = 0;
-    for (uint32_t t0 = 0; t0 < count; t0 += SLOTS * SETS) {
+// Pairs in reach wait in the warp's queue until there is one for every lane.
+template <typename TOUR, typename SH>
+struct NearQueue {
+    const TOUR& T;
+    typename SH::Reach& q;
+    NearBest& nb;
+    uint32_t z;
+    uint32_t count = 0;
+
+    // SETS times 32 of the queue's last entries, fewer at the end
+    template <int SETS>
+    __device__ __forceinline__ void take() {
+        const uint32_t lane = threadIdx.x & 31;
         uint32_t j[SETS], p[SETS];
-        float ej[SETS], en[SETS], s[SETS];
+        float s[SETS];
         bool in[SETS];
+        const uint32_t from = count > 32u * SETS ? count - 32u * SETS : 0u;
 #pragma unroll
         for (int u = 0; u < SETS; ++u) {
-            const uint32_t t = t0 + SLOTS * u + lane / WIDTH;
-            in[u] = t < count && k < T.kc;
-            j[u] = from[min(t, count - 1)];
+            const uint32_t t = from + 32 * u + lane;
+            in[u] = t < count;
+            j[u] = q.j[in[u] ? t : 0];
+            p[u] = q.p[in[u] ? t : 0];
+            s[u] = q.s[in[u] ? t : 0];
         }
+        if constexpr (sizeof(typename TOUR::Index) == 4) {
 #pragma unroll
-        for (int u = 0; u < SETS; ++u) {
-            const uint32_t jn = T.wrap(j[u] + 1);
-            ej[u] = j[u] == z ? kNoEdge : T.E[j[u]];
-            en[u] = jn == z ? kNoEdge : T.E[jn];
-            p[u] = T.pos[T.nbr[T.id[j[u]] * TOUR::kList + (in[u] ? k : 0)]];
+            for (int u = 0; u < SETS; ++u) p[u] = T.pos[p[u]];
         }
         bool met = false;
         float lowest = 0.f;
+#pragma unroll
+        for (int u = 0; u < SETS; ++u) {
+            const uint32_t jn = T.wrap(j[u] + 1);
+            const float ej = j[u] == z ? kNoEdge : T.E[j[u]], en = jn == z ? kNoEdge : T.E[jn];
+            met |= near_meet(T, in[u], j[u], p[u], s[u], ej, en, z, nb, lowest);
+        }
+        near_share(nb, met, lowest);
+        count = from;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void add(bool in, uint32_t j, uint32_t p, float s) {
+        const uint32_t lane = threadIdx.x & 31;
+        const uint32_t votes = __ballot_sync(0xffffffffu, in);
+        if (votes == 0) return;
+        if (in) {
+            const uint32_t t = count + __popc(votes & ((1u << lane) - 1u));
+            q.j[t] = (typename TOUR::Index)j;
+            q.p[t] = (typename TOUR::Index)p;
+            q.s[t] = s;
+        }
+        count += __popc(votes);
+        __syncwarp();
+        if (count > 32) take<1>();
+    }
+    __device__ __forceinline__ void rest() {
+        if (count) take<1>();
+    }
+};
+
+// Entries FIRST .. FIRST + WIDTH - 1 of the lists of `count` of the warp's slots
+// (slots w.open[0 .. count), or with FIRST == 0 all), a lane per entry and
+// 32 / WIDTH slots at a time (a long list keeps no other slot waiting), SETS
+// times that many in flight.  Pairs in reach go to the queue; the slots whose
+// entries were all in reach are left in w.open, and their number is returned.
+template <uint32_t FIRST, uint32_t WIDTH, int SETS, typename TOUR, typename SLOTS, typename QUEUE>
+__device__ __forceinline__ uint32_t near_lists(const TOUR& T, SLOTS& w, uint32_t count,
+                                               QUEUE& queue, const NearBest& nb) {
+    using IX = typename TOUR::Index;
+    constexpr uint32_t PER = 32 / WIDTH;
+    const uint32_t lane = threadIdx.x & 31, k = FIRST + lane % WIDTH;
+    uint32_t open = 0;
+    for (uint32_t t0 = 0; t0 < count; t0 += PER * SETS) {
+        uint32_t i[SETS], j[SETS], p[SETS];
+        float s[SETS];
+        bool in[SETS];
+#pragma unroll
+        for (int u = 0; u < SETS; ++u) {
+            const uint32_t t = t0 + PER * u + lane / WIDTH;
+            in[u] = t < count && k < T.kc;
+            i[u] = FIRST == 0 ? min(t, count - 1) : w.open[min(t, count - 1)];
+            j[u] = w.j[i[u]];
+            const NearEntry<IX> e = T.nbr[w.id[i[u]] * TOUR::kList + (in[u] ? k : 0)];
+            if constexpr (sizeof(IX) == 4) {
+                p[u] = e.id;
+                s[u] = e.s;
+            } else {
+                p[u] = T.pos[e.id];
+            }
+        }
         const float h = near_half(nb.B);
 #pragma unroll
         for (int u = 0; u < SETS; ++u) {
-            s[u] = near_sq(T.xy[j[u]], T.xy[p[u]]);
-            in[u] = in[u] && s[u] <= near_limit(fmaxf(ej[u], en[u]) + h);
+            if constexpr (sizeof(IX) != 4) s[u] = near_sq(T.xy[j[u]], T.xy[p[u]]);
+            in[u] = in[u] && s[u] <= near_limit(w.m[i[u]] + h);
         }
 #pragma unroll
-        for (int u = 0; u < SETS; ++u)
-            met |= near_meet(T, in[u], j[u], p[u], s[u], ej[u], en[u], z, nb, lowest);
-        near_share(nb, met, lowest);
-#pragma unroll
         for (int u = 0; u < SETS; ++u) {
-            // open <= t0 + SLOTS * u: entries still to be read are not written
+            // open <= t0 + PER * u: entries still to be read are not written
             const uint32_t ends =
                 __ballot_sync(0xffffffffu, in[u] && lane % WIDTH == WIDTH - 1);
-            if (ends >> lane & 1u)
-                out[open + __popc(ends & ((1u << lane) - 1u))] = (typename TOUR::Index)j[u];
+            if (ends >> lane & 1u) w.open[open + __popc(ends & ((1u << lane) - 1u))] = (IX)i[u];
             open += __popc(ends);
+            queue.add(in[u], j[u], p[u], s[u]);
         }
         __syncwarp();
     }
@@ -628,11 +734,12 @@ __device__ __forceinline__ uint32_t near_lists(const TOUR& T, const typename TOU
 }
 
 // One best-improvement sweep; the packed key of the best move (kNoMove if
-// none).  parity alternates from sweep to sweep (it names the result slots).
+// none).  parity alternates from sweep to sweep (it names the counters).
 //
-// With a cluster (CL) every CTA holds the same tour; the slots are dealt to all
-// of its warps (rank: this CTA's, of `ranks`), which leave their best keys in
-// every CTA's shared memory, and one cluster barrier closes the sweep.
+// near_scan is the sweep of one CTA's share: the slots are dealt to the warps of
+// `ranks` CTAs, of which this is number `rank`; each lane's best key comes back.
+// With ALL_EDGES (a tour in shared memory) large discs are replaced by the whole
+// tour's edges.
 //
 // 1. Each warp re-evaluates the best pairs that the warps met in the last
 //    sweep, where their cities are now: real pairs of this tour, and most of
@@ -643,17 +750,16 @@ __device__ __forceinline__ uint32_t near_lists(const TOUR& T, const typename TOU
 //    each, or a part of one where there are fewer discs than warps.  They wait
 //    until every list has been looked at because a disc costs what its radius
 //    says and the radius shrinks with the bound, which the CTA's warps share.
-// 4. Large discs (long edges of a tour far from a local optimum: the bound is
-//    large then, and most edges too short) are put off to all warps of the
-//    CTA, which go over all edges that can take part instead.
-template <int NT, bool CL, typename TOUR, typename SH>
-__device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
-                                                         NearSeed& seed, uint32_t parity,
-                                                         uint32_t rank = 0, uint32_t ranks = 1) {
+// 4. Large discs are put off to all warps of the CTA, which take a part each, or
+//    with ALL_EDGES go over the edges that can take part instead (long edges of
+//    a tour far from a local optimum: the bound is large then, and most edges
+//    too short).
+template <int NT, bool ALL_EDGES, typename TOUR, typename SH>
+__device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSeed& seed,
+                                              uint32_t parity, uint32_t rank, uint32_t ranks) {
     using IX = typename TOUR::Index;
     constexpr int NW = NT / 32;
     const uint32_t n = T.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (n < 4) return kNoMove;
     const uint32_t z = T.closing();
     NearBest nb{kNoMove, -1.f};
     {
@@ -673,7 +779,8 @@ __device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
         }
         near_share(nb, met, lowest);
     }
-    IX* scr = S.scratch[warp];
+    auto& w = S.slots[warp];
+    NearQueue<TOUR, SH> queue{T, S.reach[warp], nb, z};
     // the bound that the CTA's warps share
     auto exchange = [&] {
         const float shared = (float)*(volatile int*)&S.bound[parity];
@@ -685,7 +792,7 @@ __device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
         if (lane == 0) at = atomicAdd(&S.big[parity], 1u);
         at = __shfl_sync(0xffffffffu, at, 0);
         if (at >= kNearWide)
-            near_far(T, j, z, ~0u, nb);  // no room to wait
+            near_far(T, j, z, ~0u, nb.B, nb);  // no room to wait
         else if (lane == 0)
             S.wide[at] = (IX)j;
     };
@@ -696,37 +803,46 @@ __device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
     for (uint32_t base = (warp * ranks + rank) * turn; base < n; base += warps * turn) {
         const uint32_t j = base + lane;
         bool take = false;
+        float m = 0.f;
         if (lane < turn && j < n) {
             const uint32_t jn = T.wrap(j + 1);
             const float ej = j == z ? kNoEdge : T.E[j], en = jn == z ? kNoEdge : T.E[jn];
-            take = 2.f * fmaxf(ej, en) + 8.f >= -nb.B;
+            m = fmaxf(ej, en);
+            take = 2.f * m + 8.f >= -nb.B;
         }
         const uint32_t votes = __ballot_sync(0xffffffffu, take);
         if (votes == 0) continue;
-        if (take) scr[__popc(votes & ((1u << lane) - 1u))] = (IX)j;
+        if (take) {
+            const uint32_t t = __popc(votes & ((1u << lane) - 1u));
+            w.j[t] = (IX)j;
+            w.id[t] = T.id[j];
+            w.m[t] = m;
+        }
         __syncwarp();
-        uint32_t open = near_lists<0, 8, 2>(T, scr, __popc(votes), scr, z, nb);
+        uint32_t open = near_lists<0, 8, 2>(T, w, __popc(votes), queue, nb);
         if (open) {
             if constexpr (TOUR::kList == 16)
-                open = near_lists<8, 8, 1>(T, scr, open, scr, z, nb);
+                open = near_lists<8, 8, 1>(T, w, open, queue, nb);
             else
-                open = near_lists<8, 32, 2>(T, scr, open, scr, z, nb);
+                open = near_lists<8, 32, ALL_EDGES ? 2 : 4>(T, w, open, queue, nb);
         }
+        queue.rest();
         if (open && !T.whole) {
             uint32_t at = 0;
             if (lane == 0) at = atomicAdd(&S.fars[parity], open);
             at = __shfl_sync(0xffffffffu, at, 0);
-            if (lane < open && at + lane < kNearFar) S.far[at + lane] = scr[lane];
+            if (lane < open && at + lane < kNearFar) S.far[at + lane] = w.j[w.open[lane]];
             for (uint32_t o = at < kNearFar ? kNearFar - at : 0u; o < open; ++o)
-                near_far(T, scr[o], z, ~0u, nb);  // no room to wait
+                near_far(T, w.j[w.open[o]], z, ~0u, nb.B, nb);  // no room to wait
             __syncwarp();
         }
         exchange();
     }
     __syncthreads();
     const uint32_t fars = min(S.fars[parity], kNearFar);  // the same for every thread
+    const float list_bound = (float)S.bound[parity];     // likewise: final since the barrier
+    nb.B = fminf(nb.B, list_bound);
     if (fars) {
-        exchange();
         uint32_t parts = 1;
         while (2 * parts * fars <= NW) parts *= 2;
         for (uint32_t t = warp / parts; t < fars; t += NW / parts) {
@@ -734,19 +850,22 @@ __device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
             const float ej = j == z ? kNoEdge : T.E[j], en = jn == z ? kNoEdge : T.E[jn];
             const float m = fmaxf(ej, en);
             // still too short a list?
-            if (2.f * m + 8.f < -nb.B ||
-                near_sq(T.xy[j], T.xy[T.pos[T.nbr[T.id[j] * TOUR::kList + TOUR::kList - 1]]]) >
-                    near_limit(m + near_half(nb.B)))
-                continue;
+            if (2.f * m + 8.f < -nb.B || T.last_sq(j) > near_limit(m + near_half(nb.B))) continue;
             const uint32_t part = warp % parts;
-            if (near_far(T, j, z, parts * kNearDisc, nb, part, parts) && part == 0) put_off(j);
+            // (part 0 decides for all parts: the size depends on list_bound alone)
+            if (near_far(T, j, z, parts * kNearDisc, list_bound, nb, part, parts) && part == 0)
+                put_off(j);
         }
-        exchange();
+        if (lane == 0 && nb.B < list_bound) atomicMin(&S.far_bound[parity], (int)nb.B);
     }
     __syncthreads();
     const uint32_t big = min(S.big[parity], kNearWide);  // the same for every thread
-    if (big) {
-        nb.B = fminf(nb.B, (float)S.bound[parity]);
+    const float bound = fminf(list_bound, (float)S.far_bound[parity]);
+    nb.B = fminf(nb.B, bound);
+    if (!ALL_EDGES) {
+        for (uint32_t o = 0; o < big; ++o)
+            near_far(T, S.wide[o], z, ~0u, bound, nb, warp, NW);
+    } else if (big) {
         for (uint32_t base = warp * 32; base < n; base += NT) {  // whole warps
             const uint32_t g = base + lane;
             const bool take = g < n && g != z && 2.f * T.E[g] + 8.f >= -nb.B;
@@ -773,9 +892,38 @@ __device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
             }
         }
     }
-    // every warp's key to every CTA, then the minimum
-    const uint64_t best = warp_min_u64(nb.key);
-    const uint32_t mine = rank * NW + warp;
+    return nb.key;
+}
+
+// A lane's share of the warps' keys and its seed for the next sweep; the best
+// key, in every lane.
+template <typename TOUR>
+__device__ __forceinline__ uint64_t near_pick(const TOUR& T, const unsigned long long* keys,
+                                              uint32_t count, NearSeed& seed) {
+    uint64_t k = kNoMove;
+    for (uint32_t w = threadIdx.x & 31; w < count; w += 32) {
+        const uint64_t o = *(volatile const unsigned long long*)&keys[w];
+        k = o < k ? o : k;
+    }
+    seed.a = seed.b = 0;
+    if (k != kNoMove) {
+        seed.a = T.id[T.slot(key_i(k))];
+        seed.b = T.id[T.slot(key_j(k))];
+    }
+    return warp_min_u64(k);
+}
+
+// The sweep of one CTA, or of a cluster (CL) whose CTAs all hold the same tour:
+// the warps leave their best keys in every CTA's shared memory, and one cluster
+// barrier closes the sweep.
+template <int NT, bool CL, typename TOUR, typename SH>
+__device__ __forceinline__ uint64_t near_sweep(const TOUR& T, SH& S, NearSeed& seed,
+                                               uint32_t parity, uint32_t rank = 0,
+                                               uint32_t ranks = 1) {
+    constexpr int NW = NT / 32;
+    const uint32_t lane = threadIdx.x & 31, mine = rank * NW + (threadIdx.x >> 5);
+    if (T.n < 4) return kNoMove;
+    const uint64_t best = warp_min_u64(near_scan<NT, true>(T, S, seed, parity, rank, ranks));
     if constexpr (CL) {
         if (lane < ranks) cluster_store(&S.wbest[parity][mine], lane, best);
     } else {
@@ -788,17 +936,7 @@ __device__ __forceinline__ unsigned long long near_sweep(const TOUR& T, SH& S,
     } else {
         __syncthreads();
     }
-    uint64_t k = kNoMove;
-    for (uint32_t w = lane; w < ranks * NW; w += 32) {
-        const uint64_t o = S.wbest[parity][w];
-        k = o < k ? o : k;
-    }
-    seed.a = seed.b = 0;
-    if (k != kNoMove) {
-        seed.a = T.id[T.slot(key_i(k))];
-        seed.b = T.id[T.slot(key_j(k))];
-    }
-    return warp_min_u64(k);
+    return near_pick(T, S.wbest[parity], ranks * NW, seed);
 }
 
 }  // namespace logo

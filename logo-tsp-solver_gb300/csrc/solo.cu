@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(NT) near_solo_kernel(SoloArgs A) {
     T.E = reinterpret_cast<float*>(smem_raw + l.e);
     T.id = reinterpret_cast<uint32_t*>(smem_raw + l.id);
     T.pos = reinterpret_cast<uint32_t*>(smem_raw + l.pos);
-    T.nbr = A.near.nbr;
+    T.nbr = reinterpret_cast<NearEntry<uint32_t>*>(A.near.nbr);
     T.cell = A.near.cell;
     T.cellid = A.near.cellid;
     T.g = A.near.g;
@@ -234,7 +234,8 @@ __global__ void near_scatter_kernel(const float2* __restrict__ xy, uint32_t n, N
 
 __global__ void near_lists_kernel(const float2* __restrict__ xy, uint32_t n, NearIndex I) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n) near_search<uint32_t, kCtxNear>(v, xy, I.g, I.cell, I.cellid, I.nbr);
+    if (v < n) near_search<uint32_t, kCtxNear>(v, xy, I.g, I.cell, I.cellid,
+                                                reinterpret_cast<NearEntry<uint32_t>*>(I.nbr));
 }
 
 void solo_config(uint32_t n, int nt, uint32_t ctas, cudaLaunchConfig_t* cfg,
@@ -308,19 +309,19 @@ cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s) {
 
 size_t near_index_words(uint32_t n) {
     // lists (also the sort's counters), cells and their end, cities by cell
-    return std::max<size_t>((size_t)n * kCtxNear, near_cells_max(n)) + near_cells_max(n) + 1 + n;
+    return std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n)) + near_cells_max(n) + 1 + n;
 }
 
 void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n) {
-    I.nbr = words;
-    I.cell = I.nbr + std::max<size_t>((size_t)n * kCtxNear, near_cells_max(n));
+    I.nbr = reinterpret_cast<uint2*>(words);
+    I.cell = words + std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n));
     I.cellid = I.cell + near_cells_max(n) + 1;
 }
 
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s) {
     const uint32_t cells = (uint32_t)I.g.gx * (uint32_t)I.g.gy;
     const uint32_t grid = (n + 255) / 256;
-    uint32_t* count = I.nbr;
+    uint32_t* count = reinterpret_cast<uint32_t*>(I.nbr);
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t) * cells, s);
     if (e != cudaSuccess) return e;
     near_count_kernel<<<grid, 256, 0, s>>>(xy, n, I.g, count);

@@ -92,3 +92,26 @@ def test_one_cluster_and_graph_agree(lg, inst, n):
         res.append((t, tr, st["sweeps"], u, su["final_length"], su["moves"], su["sweeps"]))
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,kind", [(6145, "uniform"), (6999, "heaps"), (7000, "clumps"),
+                                    (8000, "line"), (9001, "lattice"), (20011, "uniform")])
+def test_grid_and_graph_agree(lg, inst, n, kind):
+    """Above the cluster's sizes, the grid-wide launch against the graph-driven
+    descent: every move, a bounded descent that goes on, and an ILS call."""
+    xy = points(inst, kind, n, 60 + n)
+    r = lg.nn_tour(xy)
+    res = []
+    for mode in (lg.DESCENT_GRAPH, lg.DESCENT_AUTO):
+        with lg.Solver(xy) as s:
+            s.set_descent_mode(mode)
+            s.set_route(r)
+            st = s.descend_resident(max_moves=5)
+            mid = s.get_route()
+            t, tr, sd = s.optimize_trace(mid, max_moves=400)
+            u, su = s.ils(t, 2, 5, n % 2)
+            step = s.optimize_step(u)
+        res.append((st["moves"], st["sweeps"], mid, t, tr, sd["sweeps"], u, su["final_length"],
+                    su["moves"], su["sweeps"], su["accepted"], step))
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
