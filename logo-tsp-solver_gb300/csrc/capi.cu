@@ -183,13 +183,13 @@ SoloArgs solo_args(const logo_ctx* c) {
     A.near = c->near;
     A.Qbest = c->d_Qbest;
     A.route_best = c->d_route_best;
+    A.pos = c->d_pos;
     return A;
 }
 
 GridArgs grid_args(const logo_ctx* c) {
     GridArgs A{};
     A.solo = solo_args(c);
-    A.pos = c->d_pos;
     A.gs = c->d_grid;
     return A;
 }
@@ -575,6 +575,59 @@ logo_status poisoned_error(logo_ctx* c) {
     return fail(c, LOGO_ERR_DEVICE_FAULT,
                 "context unusable: a device-side wait timed out earlier; destroy it and "
                 "create a new one");
+}
+
+logo_status status_to_error(logo_ctx* c, unsigned int st);
+bool use_solo(const logo_ctx* c);
+bool use_grid(const logo_ctx* c);
+std::mutex& coop_lock(int device);
+
+// A descent of the caller's route, or with step one sweep of it, as one launch
+// (the context's use_solo or use_grid holds): the launch loads and checks the
+// route and leaves the state in h_st, so the host waits once.  *stored: the
+// resulting tour has gone to `out` (direct mode).
+logo_status whole_call(logo_ctx* c, const uint32_t* route, uint32_t* out,
+                       unsigned long long max_moves, bool step, bool lengths, bool* stored) {
+    if (!route) return fail(c, LOGO_ERR_INVALID_ARG, "route is NULL");
+    WholeCall call{};
+    call.src = route;
+    call.out = out && route_direct(c) ? out : nullptr;
+    if (stored) *stored = call.out != nullptr;
+    if (!route_direct(c)) {
+        CK(c, cudaMemcpyAsync(c->d_route[0], route, sizeof(uint32_t) * c->n,
+                              cudaMemcpyHostToDevice, c->stream));
+        call.src = c->d_route[0];
+    }
+    if (++c->load_epoch == 0xFFFFFFFFu) {  // every value seen holds is stale again
+        CK(c, cudaMemsetAsync(c->d_seen, 0, sizeof(uint32_t) * c->n, c->stream));
+        c->load_epoch = 1;
+    }
+    call.mirror = c->h_st;
+    call.max_moves = max_moves;
+    call.seen = c->d_seen;
+    call.epoch = c->load_epoch;
+    call.step = step;
+    call.lengths = lengths;
+    c->have_route = false;
+    std::unique_lock<std::mutex> lk;
+    if (use_solo(c)) {
+        SoloArgs A = solo_args(c);
+        A.call = call;
+        CK(c, launch_solo(A, false, c->solo_ctas, c->stream));
+    } else {
+        GridArgs A = grid_args(c);
+        A.solo.call = call;
+        lk = std::unique_lock<std::mutex>(coop_lock(c->device));
+        CK(c, launch_near_grid(A, false, c->grid_ctas, c->stream));
+    }
+    ++c->host_waits;
+    CK(c, cudaStreamSynchronize(c->stream));
+    if (c->h_st->bad_route)
+        return fail(c, LOGO_ERR_INVALID_ARG, "route is not a permutation of 0..n-1");
+    c->have_route = true;
+    const unsigned int st = c->h_st->status & ~kErrMoveLimit;
+    if (st) return status_to_error(c, st);
+    return LOGO_OK;
 }
 
 logo_status status_to_error(logo_ctx* c, unsigned int st) {
@@ -1166,10 +1219,29 @@ logo_status logo_get_route(logo_ctx* c, uint32_t* route) {
 
 static logo_status sweep_once(logo_ctx* c, logo_move* out, bool reset_enqueued);
 
+static void report_move(const logo_ctx* c, logo_move* out) {
+    const uint64_t k = c->h_st->best_key;
+    if (k == kNoMove) {
+        out->i = 0;
+        out->j = 0;
+        out->minchange = 0;
+    } else {
+        out->i = key_i(k);
+        out->j = key_j(k);
+        out->minchange = key_delta(k);
+    }
+}
+
 logo_status logo_best_move(logo_ctx* c, const uint32_t* route, logo_move* out) {
     if (!c || !out) return LOGO_ERR_INVALID_ARG;
     if (c->poisoned) return poisoned_error(c);
     CK(c, cudaSetDevice(c->device));
+    if (!c->own_kernel && (use_solo(c) || use_grid(c))) {
+        const logo_status w = whole_call(c, route, nullptr, ~0ull >> 1, true, false, nullptr);
+        if (w != LOGO_OK) return w;
+        report_move(c, out);
+        return LOGO_OK;
+    }
     logo_status s = upload_route(c, route, ~0ull >> 1);
     if (s != LOGO_OK) return s;
     return sweep_once(c, out, true);
@@ -1190,16 +1262,7 @@ static logo_status sweep_once(logo_ctx* c, logo_move* out, bool reset_enqueued) 
     logo_status s = read_state(c);
     if (s != LOGO_OK) return s;
     if (c->h_st->status) return status_to_error(c, c->h_st->status);
-    const uint64_t k = c->h_st->best_key;
-    if (k == kNoMove) {
-        out->i = 0;
-        out->j = 0;
-        out->minchange = 0;
-    } else {
-        out->i = key_i(k);
-        out->j = key_j(k);
-        out->minchange = key_delta(k);
-    }
+    report_move(c, out);
     return LOGO_OK;
 }
 
@@ -1247,6 +1310,25 @@ static logo_status descend_impl(logo_ctx* c, uint32_t* route, uint64_t max_moves
     if (c->poisoned) return poisoned_error(c);
     CK(c, cudaSetDevice(c->device));
     Timer t(c, stats != nullptr);  // no stats: no timing and no extra wait
+    if (!(trace && trace_cap) && (use_solo(c) || use_grid(c))) {
+        bool stored = false;
+        logo_status s = whole_call(c, route, route, max_moves ? max_moves : ~0ull >> 1, false,
+                                   stats != nullptr, &stored);
+        if (s == LOGO_OK && !stored) s = download_route(c, route, false);
+        const double ms = t.stop();
+        if (s != LOGO_OK) return s;
+        if (stats) {
+            std::memset(stats, 0, sizeof(*stats));
+            stats->moves = c->h_st->moves;
+            stats->sweeps = c->h_st->sweeps - c->h_st->sweeps_at_reset;
+            stats->pair_evals = pair_evals_of(c, stats->sweeps, 0);
+            stats->descents = 1;
+            stats->start_length = c->h_st->start_length;
+            stats->final_length = c->h_st->length;
+            stats->device_ms = ms;
+        }
+        return LOGO_OK;
+    }
     // without stats or a trace nothing runs between the load and the descent:
     // the load also resets the descent, and in direct route mode the result
     // is written back before the one final wait

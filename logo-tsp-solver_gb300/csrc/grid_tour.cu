@@ -12,7 +12,19 @@
 // arrays are read through it, and other SMs rewrite them between barriers;
 // bounded by %globaltimer, after which the CTA sets kErrTimeout and every CTA
 // gives up in turn).  Every CTA reads the same keys and so does the same.
-#include <mutex>
+//
+// As a whole call the launch also loads and checks the caller's route and leaves
+// result and state in host memory: one launch and one wait (best move and move
+// of a 100,000-city route: 111 -> 60 us; best move of 1,000,000: 612 -> 168 us,
+// most of it the route's way from host memory).
+//
+// Discs of more than kGridDisc cities (long edges of a tour far from a local
+// optimum) are put off to all CTAs: the few edges against every edge that can
+// take part, after one more barrier.  One CTA going through them held up the rest
+// (best move of the 1,000,000-city tour: 375 us).  Dealing out every slot
+// whose list was too short the same way costs the barrier in each sweep and was
+// slower (n = 20,000: 18.9 -> 20.8 us a sweep).
+#include <cstddef>
 
 #include "logo_device.cuh"
 #include "logo_internal.h"
@@ -80,6 +92,56 @@ __device__ __forceinline__ void grid_place(GridTour& T, const uint32_t* route, c
     }
 }
 
+// The pairs of `count` edges with every edge, by `threads` threads.
+__device__ __forceinline__ void grid_edges(const GridTour& T, const uint32_t* edges,
+                                           uint32_t count, uint32_t z, NearBest& nb, uint32_t tid,
+                                           uint32_t threads) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t base = tid - lane; base < T.n; base += threads) {  // whole warps
+        const uint32_t g = base + lane;
+        near_edges(T, edges, count,
+                   g < T.n && g != z && 2.f * T.E[min(g, T.n - 1)] + 8.f >= -nb.B, g, z, nb);
+    }
+}
+
+// The caller's route as grid_place, with the check that it is a permutation
+// (load_route_kernel in tour.cu) and the tour's other copy; true when this
+// thread met a city twice or none.
+__device__ __forceinline__ bool grid_load(GridTour& T, const SoloArgs& A,
+                                          unsigned long long* length, uint32_t tid,
+                                          uint32_t threads) {
+    const uint32_t n = T.n, lane = threadIdx.x & 31;
+    T.o = 0;
+    T.rev = false;
+    bool bad = false;
+    unsigned long long sum = 0;
+    for (uint32_t base = tid - lane; base < n; base += threads) {  // whole warps
+        const uint32_t k = base + lane;
+        uint32_t v = k < n ? A.call.src[k] : 0u;
+        uint32_t w = __shfl_up_sync(0xffffffffu, v, 1);
+        if (lane == 0) w = A.call.src[k == 0 ? n - 1 : k - 1];
+        if (k >= n) continue;
+        const bool miss = v >= n || atomicExch(&A.call.seen[v], A.call.epoch) == A.call.epoch;
+        bad |= miss;
+        if (A.R0 != A.call.src) A.R0[k] = v;
+        v = min(v, n - 1);
+        w = min(w, n - 1);
+        const float2 p = A.xy[v];
+        const float e = near_dist(A.xy[w], p);
+        A.Q0[k] = OrderedCity{p.x, p.y, e, 0.f};
+        T.xy[k] = p;
+        T.E[k] = e;
+        T.id[k] = v;
+        T.pos[v] = k;
+        sum += (unsigned long long)e;
+    }
+    if (length) {
+        sum = warp_sum_u64(sum);
+        if (lane == 0 && sum) atomicAdd(length, sum);
+    }
+    return bad;
+}
+
 template <bool ILS>
 __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     constexpr int NT = kGridNT, NW = NT / 32;
@@ -87,13 +149,15 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     __shared__ bool bar_ok;
     __shared__ uint2 seeds[32];
     __shared__ unsigned long long best_key;
+    __shared__ uint32_t wide_count;
     DevState* st = A.solo.st;
+    const bool whole = !ILS && A.solo.call.src != nullptr;
     // set before the launch and identical for every CTA
-    if (*(volatile unsigned int*)&st->converged) return;
+    if (!whole && *(volatile unsigned int*)&st->converged) return;
     const uint32_t n = A.solo.n, rank = blockIdx.x, ranks = gridDim.x;
     const uint32_t tid = rank * NT + threadIdx.x, threads = ranks * NT;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t cur = *(volatile unsigned int*)&st->cur;
+    const uint32_t cur = whole ? 0u : *(volatile unsigned int*)&st->cur;
     OrderedCity* Qg = cur ? A.solo.Q1 : A.solo.Q0;
     uint32_t* Rg = cur ? A.solo.R1 : A.solo.R0;
     // the ring lies in the other tour buffer: xy, E, id by slot
@@ -105,19 +169,61 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     T.xy = reinterpret_cast<float2*>(ring);
     T.E = reinterpret_cast<float*>(ring + 8 * (size_t)n);
     T.id = reinterpret_cast<uint32_t*>(ring + 12 * (size_t)n);
-    T.pos = A.pos;
+    T.pos = A.solo.pos;
     T.nbr = reinterpret_cast<NearEntry<uint32_t>*>(A.solo.near.nbr);
     T.cell = A.solo.near.cell;
     T.cellid = A.solo.near.cellid;
     T.g = A.solo.near.g;
     GridBarrier barrier{A.gs, st, &bar_ok};
     S.init();
-    grid_place(T, Rg, A.solo.xy, tid, threads);
-    bool ok = barrier();
-    NearSeed seed;
+    // this CTA's best key, and the counters of the next sweep
     uint32_t parity = 0;
-    unsigned long long m0 = *(volatile unsigned long long*)&st->moves;
-    const unsigned long long maxm = *(volatile unsigned long long*)&st->max_moves;
+    auto publish = [&](unsigned long long* keys, uint64_t key) {
+        const uint64_t mine = warp_min_u64(key);
+        if (lane == 0) S.wbest[0][warp] = mine;
+        __syncthreads();
+        if (warp == 0) {
+            const uint64_t best = warp_min_u64(lane < NW ? S.wbest[0][lane] : kNoMove);
+            if (lane == 0) {
+                keys[rank] = best;
+                S.reset(parity ^ 1);
+            }
+        }
+    };
+    // a whole call's state goes to the host with the last CTA, so that a wait of any
+    // CTA that ran out is in it
+    auto leave = [&] {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            bar_ok = atomicAdd(&A.gs->left, 1u) == ranks - 1;
+            __threadfence();
+        }
+        __syncthreads();
+        if (bar_ok) leave_call(st, A.solo.call.mirror);
+    };
+    const bool step = whole && A.solo.call.step, lengths = whole && A.solo.call.lengths;
+    if (whole && tid == 0) start_call(st, A.solo.call.max_moves);
+    if (whole) {
+        if (grid_load(T, A.solo, lengths ? &A.gs->start_length : nullptr, tid, threads))
+            atomicExch(&A.gs->bad, 1ull);
+    } else {
+        grid_place(T, Rg, A.solo.xy, tid, threads);
+    }
+    bool ok = barrier();
+    if (whole && ok && ld_acquire_u64(&A.gs->bad)) {  // the same in every CTA
+        if (tid == 0) {
+            st->bad_route = 1;
+            st->converged = 1;
+        }
+        leave();
+        return;
+    }
+    NearSeed seed;
+    unsigned long long m0 = whole ? 0ull : *(volatile unsigned long long*)&st->moves;
+    const unsigned long long maxm =
+        whole ? A.solo.call.max_moves : *(volatile unsigned long long*)&st->max_moves;
+    unsigned long long step_key = kNoMove;
     unsigned long long m = 0, sweeps = 0, total_m = 0;
     unsigned long long best_len = 0, accepted = 0, kicks = 0;
     uint64_t rng = 0;
@@ -129,32 +235,88 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     for (uint32_t it = 0; ok; ++it) {
         m = 0;
         for (;;) {
-            const uint64_t mine =
-                warp_min_u64(near_scan<NT, false>(T, S, seed, parity, rank, ranks));
-            if (lane == 0) S.wbest[0][warp] = mine;
+            NearBest nb{near_scan<NT, false>(T, S, seed, parity, rank, ranks), -1.f};
+            const uint32_t z = T.closing();
             __syncthreads();
-            if (warp == 0) {
-                const uint64_t best = warp_min_u64(lane < NW ? S.wbest[0][lane] : kNoMove);
-                if (lane == 0) {
-                    A.gs->keys[parity][rank] = best;
-                    S.reset(parity ^ 1);  // the next sweep's
+            const uint32_t huges = S.huges[parity];  // the same for every thread
+            if (huges) {
+                // the edges of these slots that reach beyond their lists
+                if (nb.key != kNoMove) nb.B = (float)key_delta(nb.key);
+                const float h = near_half((float)S.bound[parity]);
+                for (uint32_t o = warp; o < 2 * huges; o += NW) {
+                    const uint32_t j = S.huge[o / 2], f = o & 1 ? T.wrap(j + 1) : j;
+                    if (f == z || T.last_sq(j) > near_limit(T.E[f] + h)) continue;
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(&A.gs->wides[parity], 1u);
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if (at >= kGridWide)
+                        near_far(T, j, z, ~0u, nb.B, nb);  // no room for this one
+                    else if (lane == 0)
+                        A.gs->wide[parity][at] = f;
                 }
             }
+            publish(A.gs->keys[parity], nb.key);
             if (!(ok = barrier())) break;
             ++sweeps;
+            if (tid == 0) A.gs->wides[parity ^ 1] = A.gs->takers[parity ^ 1] = 0;  // the next sweep's
             // one warp per CTA reads the keys (all of them reading the same few
             // lines queued up at L2 for 7 us)
             if (warp == 0) {
+                const uint32_t w = *(volatile uint32_t*)&A.gs->wides[parity];
                 const uint64_t k = near_pick(T, A.gs->keys[parity], ranks, seed);
                 seeds[lane] = make_uint2(seed.a, seed.b);
-                if (lane == 0) best_key = k;
+                if (lane == 0) {
+                    best_key = k;
+                    wide_count = w;
+                }
             }
             __syncthreads();
-            const uint64_t key = best_key;
+            uint64_t key = best_key;
+            const uint32_t wides = min(wide_count, kGridWide);
+            if (wides) {
+                // edges put off, with every edge that can take part: listed first,
+                // so that the pairs can be dealt evenly, unless those are too many
+                NearBest more{key, key == kNoMove ? -1.f : (float)key_delta(key)};
+                for (uint32_t base = tid - lane; base < n; base += threads) {
+                    const uint32_t g = base + lane;
+                    const bool takes = g < n && g != z && 2.f * T.E[g] + 8.f >= -more.B;
+                    const uint32_t votes = __ballot_sync(0xffffffffu, takes);
+                    if (votes == 0) continue;
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(&A.gs->takers[parity], (uint32_t)__popc(votes));
+                    at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1u));
+                    if (takes && at < kGridTakers) A.gs->taker[at] = g;
+                }
+                if (!(ok = barrier())) break;
+                const uint32_t takers = *(volatile uint32_t*)&A.gs->takers[parity];
+                if (takers <= kGridTakers) {
+                    for (uint32_t base = tid - lane; base < wides * takers; base += threads) {
+                        const uint32_t t = base + lane;
+                        const bool in = t < wides * takers;
+                        near_edges(T, &A.gs->wide[parity][in ? t / takers : 0], 1u, in,
+                                   A.gs->taker[in ? t % takers : 0], z, more);
+                    }
+                } else {
+                    grid_edges(T, A.gs->wide[parity], wides, z, more, tid, threads);
+                }
+                publish(A.gs->wide_keys[parity], more.key);
+                if (!(ok = barrier())) break;
+                if (warp == 0) {
+                    NearSeed other;
+                    const uint64_t k = near_pick(T, A.gs->wide_keys[parity], ranks, other);
+                    if (lane == 0) best_key = k;
+                }
+                __syncthreads();
+                key = best_key;
+            }
             seed.a = seeds[lane].x;
             seed.b = seeds[lane].y;
             parity ^= 1u;
             if (key == kNoMove) break;  // local optimum
+            if (step) {
+                step_key = key;
+                break;
+            }
             // reported move (i, j+1): p = i < q = j+1 (twoOptLocalSolver.cpp:41-48)
             const uint32_t p = key_i(key), q = key_j(key);
             if (!(p >= 1 && q < n && q >= p + 2)) {
@@ -217,25 +379,37 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
         ++kicks;
         m0 = 0;
     }
-    if (ok) {
+    if (ok && !step) {  // (a step's tour went there as it was loaded)
         // the tour in its order, with the positions that other kernels keep
+        unsigned long long part = 0;
         for (uint32_t k = tid; k < n; k += threads) {
             const uint32_t j = T.slot(k);
             const uint32_t id = T.id[j];
             const float2 c = T.xy[j];
             const OrderedCity o{c.x, c.y, T.E[T.rev ? T.wrap(j + 1) : j], 0.f};
+            part += (unsigned long long)o.e;
             Rg[k] = id;
             Qg[k] = o;
             T.pos[id] = k;
             if (ILS) A.solo.Qbest[k] = o;
+            if (whole && A.solo.call.out) A.solo.call.out[k] = id;
         }
+        if (lengths) {
+            part = warp_sum_u64(part);
+            if (lane == 0 && part) atomicAdd(&A.gs->length[0], part);
+            ok = barrier();
+        }
+    }
+    if (lengths && tid == 0) {
+        st->start_length = ld_acquire_u64(&A.gs->start_length);
+        st->length = ld_acquire_u64(&A.gs->length[0]);
     }
     if (tid == 0) {
         if (ok) {
             st->moves = m0 + m;
             st->total_moves += total_m;
-            st->sweeps += sweeps;
-            st->best_key = kNoMove;
+            if (!step) st->sweeps += sweeps;
+            st->best_key = step_key;
             if (ILS) {
                 st->rng = rng;
                 st->best_length = best_len;
@@ -245,8 +419,9 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             if (limit) atomicOr(&st->status, kErrMoveLimit);
             if (bad) atomicOr(&st->status, kErrBadKey);
         }
-        st->converged = 1;
+        st->converged = step && ok ? 0u : 1u;
     }
+    if (whole) leave();
 }
 
 template <bool ILS>
@@ -268,7 +443,7 @@ int near_grid_ctas(uint32_t n, int device) {
 }
 
 cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t s) {
-    const cudaError_t e = cudaMemsetAsync(A.gs, 0, sizeof(GridSync), s);
+    const cudaError_t e = cudaMemsetAsync(A.gs, 0, offsetof(GridSync, wide_keys), s);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);

@@ -176,6 +176,32 @@ __host__ __device__ __forceinline__ uint32_t oropt_src(uint32_t k, uint32_t s, u
     return k - L;
 }
 
+// ---- whole calls -----------------------------------------------------------------
+// What a route load that also prepares a descent of at most max_moves moves
+// leaves (load_route_kernel in tour.cu); one thread.
+__device__ __forceinline__ void start_call(DevState* st, unsigned long long max_moves) {
+    st->bad_route = 0u;
+    st->cur = 0u;
+    st->best_key = kNoMove;
+    for (int v = 0; v < kOrSlots; ++v) st->or_key[v] = kNoMove;
+    st->moves = 0;
+    st->nbr_sweeps = 0;
+    st->status = 0u;
+    st->converged = 0u;
+    st->sweeps_at_reset = st->sweeps;
+    st->max_moves = max_moves;
+}
+// Copies the state to its mirror in pinned host memory; one whole CTA, whose
+// thread 0 wrote the state.  The host reads it once the launch has completed.
+__device__ __forceinline__ void leave_call(const DevState* st, DevState* mirror) {
+    static_assert(sizeof(DevState) % sizeof(unsigned long long) == 0, "copied in words");
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < sizeof(DevState) / sizeof(unsigned long long);
+         k += blockDim.x)
+        reinterpret_cast<volatile unsigned long long*>(mirror)[k] =
+            reinterpret_cast<const volatile unsigned long long*>(st)[k];
+}
+
 // ---- programmatic dependent launch -------------------------------------------
 // Kernels of the step chain (route load, sweeps, move, route store) are
 // launched with programmatic stream serialization (launch_chained in

@@ -157,6 +157,19 @@ size_t near_index_words(uint32_t n);
 void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);  // words 8-byte aligned
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s);
 
+// A whole call as one launch: the route is loaded (and checked) by the launch
+// itself, and its state and result are left in host memory.
+struct WholeCall {
+    const uint32_t* src;   // the caller's route, or a device copy of it; null: the resident tour
+    uint32_t* out;         // where the resulting tour also goes (null: nowhere)
+    DevState* mirror;      // pinned host memory: *st as the launch leaves it
+    unsigned long long max_moves;
+    uint32_t* seen;        // grid-wide launch: the last load that met each city
+    uint32_t epoch;        // number of this load (see launch_load_route)
+    bool step;             // one sweep, no move: its key stays in st->best_key
+    bool lengths;          // also st->start_length and st->length
+};
+
 // One cluster runs a whole descent, or a whole ILS call, of a tour of 8 to
 // kSoloMaxN cities (solo.cu).
 constexpr uint32_t kSoloMaxN = 6144;
@@ -175,6 +188,8 @@ struct SoloArgs {
     uint32_t* route_best;
     uint32_t kicks;
     int kick_kind;
+    WholeCall call;  // descents only
+    uint32_t* pos;   // tour position of every city, where the context keeps it
 };
 // CTAs of the cluster for this n on the current device (0: not available).
 uint32_t solo_wanted_ctas(uint32_t n);
@@ -187,14 +202,24 @@ cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s);
 // A descent or an ILS call of a larger tour as one cooperative launch over the
 // whole device (grid_tour.cu): one CTA per SM.
 constexpr uint32_t kGridMaxCtas = 256;
+constexpr uint32_t kGridWide = 1024, kGridTakers = 8192;
 struct GridSync {
     unsigned long long arrived;    // barrier arrivals so far
     unsigned long long length[2];  // tour length of the descent in hand, by its parity
+    unsigned long long start_length;
+    unsigned long long bad;        // the route is not a permutation
+    // edges put off in a sweep, and edges that can take part in pairs with them,
+    // by its parity (more may have been offered than fit)
+    uint32_t wides[2], takers[2];
+    uint32_t left;  // CTAs that have left a whole call
+    // (set to zero up to here before a launch)
+    unsigned long long wide_keys[2][kGridMaxCtas];  // best key per CTA after those
+    uint32_t wide[2][kGridWide];
+    uint32_t taker[kGridTakers];
     unsigned long long keys[2][kGridMaxCtas];  // best key per CTA, by the sweep's parity
 };
 struct GridArgs {
-    SoloArgs solo;
-    uint32_t* pos;  // slot of every city; positions again when the launch ends
+    SoloArgs solo;  // pos: slot of every city meanwhile
     GridSync* gs;
 };
 // CTAs of the launch (0: n is not above kSoloMaxN, or not available).

@@ -152,6 +152,7 @@ struct NearTour {
 constexpr uint32_t kNearFar = 256;   // discs of a sweep's CTA that may wait for their warps
 constexpr uint32_t kNearWide = 64;   // discs that may be put off again, to the whole CTA
 constexpr uint32_t kNearDisc = 256;  // cities that a warp goes through of a disc
+constexpr uint32_t kGridDisc = 4096;  // and a CTA, where many CTAs share a tour in global memory
 
 // MAXC: CTAs that share the sweeps (a cluster, each with its own copy of the tour).
 template <int NT, int MAXC, typename IX>
@@ -164,9 +165,10 @@ struct NearShared {
     // by the sweep's parity: best delta met, entries of far and wide (more may
     // have been offered than fit)
     int bound[2], far_bound[2];  // (of its lists, and of its discs)
-    uint32_t fars[2], big[2];
+    uint32_t fars[2], big[2], huges[2];
     IX far[kNearFar];         // slots whose lists were too short
     IX wide[kNearWide];       // those of them whose discs are large
+    IX huge[kNearWide];       // and those too large for one CTA
     // each warp's slots in hand: slot, its city, its longer edge
     struct Slots {
         IX j[32], id[32], open[32];
@@ -183,7 +185,7 @@ struct NearShared {
 
     __device__ __forceinline__ void reset(uint32_t parity) {
         bound[parity] = far_bound[parity] = -1;
-        fars[parity] = big[parity] = 0;
+        fars[parity] = big[parity] = huges[parity] = 0;
     }
     // once per kernel; a barrier must follow before the first sweep
     __device__ __forceinline__ void init() {
@@ -497,6 +499,11 @@ __device__ __forceinline__ void cluster_store(unsigned long long* p, uint32_t ct
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(p)), "r"(cta));
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v) : "memory");
 }
+__device__ __forceinline__ void cluster_store(uint32_t* p, uint32_t cta, uint32_t v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(p)), "r"(cta));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                      : "memory");
@@ -683,6 +690,27 @@ struct NearQueue {
     }
 };
 
+// The pairs of `count` edges with the edges of 32 slots, a lane per slot g (in: g
+// is a slot whose edge can take part), whole warps.
+template <typename TOUR>
+__device__ __forceinline__ void near_edges(const TOUR& T, const typename TOUR::Index* edges,
+                                           uint32_t count, bool in, uint32_t g, uint32_t z,
+                                           NearBest& nb) {
+    if (!__any_sync(0xffffffffu, in)) return;
+    const uint32_t n = T.n, gs = in ? g : 0;
+    const float2 head = T.xy[gs], tail = T.xy[gs == 0 ? n - 1 : gs - 1];
+    const float eg = T.E[gs];
+    bool met = false;
+    float lowest = 0.f;
+    for (uint32_t o = 0; o < count; ++o) {
+        const uint32_t f = edges[o];
+        if (in && f != g && f != z)
+            met |= near_pair(T, f, g, near_sq(T.xy[f], head),
+                             near_sq(T.xy[f == 0 ? n - 1 : f - 1], tail), T.E[f], eg, nb, lowest);
+    }
+    near_share(nb, met, lowest);
+}
+
 // Entries FIRST .. FIRST + WIDTH - 1 of the lists of `count` of the warp's slots
 // (slots w.open[0 .. count), or with FIRST == 0 all), a lane per entry and
 // 32 / WIDTH slots at a time (a long list keeps no other slot waiting), SETS
@@ -750,10 +778,10 @@ __device__ __forceinline__ uint32_t near_lists(const TOUR& T, SLOTS& w, uint32_t
 //    each, or a part of one where there are fewer discs than warps.  They wait
 //    until every list has been looked at because a disc costs what its radius
 //    says and the radius shrinks with the bound, which the CTA's warps share.
-// 4. Large discs are put off to all warps of the CTA, which take a part each, or
-//    with ALL_EDGES go over the edges that can take part instead (long edges of
-//    a tour far from a local optimum: the bound is large then, and most edges
-//    too short).
+// 4. Large discs are put off to all warps of the CTA, which take a part each
+//    (those beyond kGridDisc stay in S.huge for the caller), or with ALL_EDGES go
+//    over the edges that can take part instead (long edges of a tour far from a
+//    local optimum: the bound is large then, and most edges too short).
 template <int NT, bool ALL_EDGES, typename TOUR, typename SH>
 __device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSeed& seed,
                                               uint32_t parity, uint32_t rank, uint32_t ranks) {
@@ -863,8 +891,10 @@ __device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSe
     const float bound = fminf(list_bound, (float)S.far_bound[parity]);
     nb.B = fminf(nb.B, bound);
     if (!ALL_EDGES) {
+        // (alike in all warps: the size depends on `bound` alone)
         for (uint32_t o = 0; o < big; ++o)
-            near_far(T, S.wide[o], z, ~0u, bound, nb, warp, NW);
+            if (near_far(T, S.wide[o], z, kGridDisc, bound, nb, warp, NW) && threadIdx.x == 0)
+                S.huge[S.huges[parity]++] = S.wide[o];
     } else if (big) {
         for (uint32_t base = warp * 32; base < n; base += NT) {  // whole warps
             const uint32_t g = base + lane;

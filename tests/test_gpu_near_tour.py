@@ -115,3 +115,30 @@ def test_grid_and_graph_agree(lg, inst, n, kind):
                     su["moves"], su["sweeps"], su["accepted"], step))
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [8, 2049, 6145, 20000])
+def test_whole_calls_and_graph_agree(lg, inst, n):
+    """A step and a bounded descent of the caller's route as one launch each,
+    from a random tour (at 20000 edges without a list of their own in nearly
+    every sweep, and more of them than are listed); a route with a city twice
+    or out of range is refused and the next call answered."""
+    xy = points(inst, "uniform", n, 80 + n)
+    r = inst.random_tour(n, 81 + n)
+    res = []
+    for mode in (lg.DESCENT_GRAPH, lg.DESCENT_AUTO):
+        with lg.Solver(xy) as s:
+            s.set_descent_mode(mode)
+            step = s.optimize_step(r)
+            for city in (r[0], n, 0xFFFFFFFF):
+                wrong = r.copy()
+                wrong[n // 2] = city
+                with pytest.raises(lg.LogoError):
+                    s.optimize_step(wrong)
+                with pytest.raises(lg.LogoError):
+                    s.optimize(wrong)
+            t, st = s.optimize(r, max_moves=12)
+            res.append((step, t, st["moves"], st["sweeps"], st["start_length"],
+                        st["final_length"], s.optimize_step(t), s.get_route()))
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
