@@ -40,7 +40,7 @@ __device__ __forceinline__ void refresh_thresholds(RowBlock<R>& rb, const Ordere
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const uint32_t i = ib + r;
-        if (i + 3 <= n) {
+        if (i >= 1 && i + 3 <= n) {  // (row 0 is no pair's)
             const int ei = (int)Q[i].e;
             rb.T[r] = (float)(B + ei) + margin;
         } else {

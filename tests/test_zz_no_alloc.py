@@ -108,3 +108,32 @@ def test_noalloc_after_a_rejected_call_and_misaligned_coordinates(lg, inst, orac
     # and the entry point still answers correctly afterwards
     got, status = _noalloc(lg, torch, xy, route)
     assert status == 0 and got == oracle_mod.best_move(xy, route)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "near", "line", "heaps", "offset", "lattice", "two"])
+def test_noalloc_windows(lg, inst, oracle_mod, kind):
+    """Around windows of 32 and tiles of 128 x 256, with windows that are out by
+    their boxes (near: an NN tour), that all tie (lattice), and where every edge
+    takes part (two: between two far clusters and back, walked densely)."""
+    torch = pytest.importorskip("torch")
+    for n in (31, 32, 33, 65, 129, 255, 256, 257, 511, 513, 1025, 2600):
+        xy = inst.uniform_f32(n, 300 + n, 1.0e4)
+        route = inst.random_tour(n, 400 + n)
+        k = np.arange(n)
+        if kind == "near":
+            route = lg.nn_tour(xy)
+        elif kind == "line":
+            xy[:, 1] = 7.0
+        elif kind == "heaps":
+            xy = np.ascontiguousarray(xy[k % 5])
+        elif kind == "offset":
+            xy = xy + np.float32(1.0e8)
+        elif kind == "lattice":
+            xy = np.stack([10.0 * (k % 50), 10.0 * (k // 50)], axis=1).astype(np.float32)
+            route = k.astype(np.uint32)
+        elif kind == "two":
+            xy = xy * np.float32(0.001)
+            xy[1::2, 0] += np.float32(1.2e6)
+            route = k.astype(np.uint32)
+        got, status = _noalloc(lg, torch, xy, route)
+        assert status == 0 and got == oracle_mod.best_move(xy, route), (n, got)
