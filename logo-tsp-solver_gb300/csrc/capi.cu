@@ -167,7 +167,7 @@ SweepLaunch sweep_args(const logo_ctx* c) {
     L.R0 = c->d_route[0];
     L.R1 = c->d_route[1];
     L.pos = c->d_pos;
-    L.nbr = c->near.nbr;
+    L.nbr = c->near.seeds;
     return L;
 }
 

@@ -108,7 +108,7 @@ constexpr uint64_t kSmallBytesPerCity = sizeof(float2) + 2 * sizeof(uint32_t);
 constexpr uint64_t kLargeLeastBytesPerCity =
     8 + 2 * 16 + 2 * 4 + 16 + 4 + 4 * (1 + kSeedNeighbours);
 constexpr uint64_t kLargeBytesPerCity =
-    kLargeLeastBytesPerCity + 8 * kCtxNear - 4 * kSeedNeighbours + 4 + 2;
+    kLargeLeastBytesPerCity + 8 * kCtxNear + 4 + 2;
 
 thread_local std::string g_server_err;
 

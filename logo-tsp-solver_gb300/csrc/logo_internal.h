@@ -61,13 +61,13 @@ struct SweepLaunch {
     uint4* work;         // ntiles entries
     uint32_t* workctl;   // tiles listed from the start, claimed, listed from the end
     // boxed variant: the tour's city ids (both buffers), the tour position of
-    // every city (kept by every kernel that moves the tour) and the context's
-    // neighbour lists (NearIndex), the pairs of whose first kSeedNeighbours
-    // entries seed the sweep's best delta
+    // every city (kept by every kernel that moves the tour) and the nearest
+    // kSeedNeighbours cities of each (NearIndex), whose pairs seed the sweep's best
+    // delta
     const uint32_t* R0;
     const uint32_t* R1;
     uint32_t* pos;
-    const uint2* nbr;
+    const uint32_t* nbr;
 };
 constexpr uint32_t kSeedNeighbours = 5;
 // k nearest other cities of every city, out[v * k + j] (construct.cpp).
@@ -150,9 +150,10 @@ struct NearIndex {
     uint2* nbr;  // kCtxNear entries per city: city, squared distance (near_tour.cuh)
     uint32_t* cell;
     uint32_t* cellid;
+    uint32_t* seeds;  // kSeedNeighbours per city: the lists' first cities (sweep.cu)
     NearGrid g;
 };
-// 32-bit words behind nbr, cell and cellid.
+// 32-bit words behind nbr, cell, cellid and seeds.
 size_t near_index_words(uint32_t n);
 void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);  // words 8-byte aligned
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s);

@@ -293,8 +293,11 @@ __global__ void near_scatter_kernel(const float2* __restrict__ xy, uint32_t n, N
 
 __global__ void near_lists_kernel(const float2* __restrict__ xy, uint32_t n, NearIndex I) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n) near_search<uint32_t, kCtxNear>(v, xy, I.g, I.cell, I.cellid,
-                                                reinterpret_cast<NearEntry<uint32_t>*>(I.nbr));
+    if (v >= n) return;
+    near_search<uint32_t, kCtxNear>(v, xy, I.g, I.cell, I.cellid,
+                                    reinterpret_cast<NearEntry<uint32_t>*>(I.nbr));
+    for (uint32_t k = 0; k < kSeedNeighbours; ++k)
+        I.seeds[(size_t)v * kSeedNeighbours + k] = I.nbr[(size_t)v * kCtxNear + min(k, n - 2)].x;
 }
 
 void solo_config(uint32_t n, int nt, uint32_t ctas, cudaLaunchConfig_t* cfg,
@@ -367,14 +370,16 @@ cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s) {
 }
 
 size_t near_index_words(uint32_t n) {
-    // lists (also the sort's counters), cells and their end, cities by cell
-    return std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n)) + near_cells_max(n) + 1 + n;
+    // lists (also the sort's counters), cells and their end, cities by cell, seeds
+    return std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n)) + near_cells_max(n) + 1 +
+           (size_t)n * (1 + kSeedNeighbours);
 }
 
 void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n) {
     I.nbr = reinterpret_cast<uint2*>(words);
     I.cell = words + std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n));
     I.cellid = I.cell + near_cells_max(n) + 1;
+    I.seeds = I.cellid + n;
 }
 
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s) {

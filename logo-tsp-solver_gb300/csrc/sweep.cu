@@ -299,7 +299,7 @@ __device__ __forceinline__ void window_reduce(float& m, float& x0, float& x1, fl
 __device__ __forceinline__ void seed_position(const OrderedCity* __restrict__ Q,
                                               const uint32_t* __restrict__ R,
                                               const uint32_t* __restrict__ pos,
-                                              const uint2* __restrict__ nbr, uint32_t n,
+                                              const uint32_t* __restrict__ nbr, uint32_t n,
                                               uint32_t i, uint64_t& best) {
     constexpr uint32_t K = kSeedNeighbours;
     // every load of the position's candidates is issued before any is used
@@ -307,7 +307,7 @@ __device__ __forceinline__ void seed_position(const OrderedCity* __restrict__ Q,
     const OrderedCity qi = Q[i], qim = Q[i >= 1 ? i - 1 : 0], qip = Q[min(i + 1, n - 1)];
     uint32_t p[K];
 #pragma unroll
-    for (uint32_t k = 0; k < K; ++k) p[k] = nbr[(size_t)t * kCtxNear + k].x;
+    for (uint32_t k = 0; k < K; ++k) p[k] = nbr[(size_t)t * K + k];
 #pragma unroll
     for (uint32_t k = 0; k < K; ++k) p[k] = min(pos[min(p[k], n - 1)], n - 1);
     OrderedCity qp[K], qpm[K], qpp[K];
@@ -346,7 +346,7 @@ __device__ __forceinline__ void seed_position(const OrderedCity* __restrict__ Q,
 __global__ void __launch_bounds__(256)
     window_seed_kernel(const OrderedCity* __restrict__ Q0, const OrderedCity* __restrict__ Q1,
                        const uint32_t* __restrict__ R0, const uint32_t* __restrict__ R1,
-                       const uint32_t* __restrict__ pos, const uint2* __restrict__ nbr,
+                       const uint32_t* __restrict__ pos, const uint32_t* __restrict__ nbr,
                        uint32_t n, float4* __restrict__ wbox, float* __restrict__ wmax,
                        float4* __restrict__ rbox, float* __restrict__ rmax,
                        uint32_t* __restrict__ workctl, uint32_t stride, DevState* st) {
