@@ -661,16 +661,43 @@ std::mutex& coop_lock(int device) {
     return locks[(unsigned)device % 64];
 }
 
+bool solo_runs(const logo_ctx* c) {
+    return c->solo_ctas > 0 && c->descent_mode != LOGO_DESCENT_GRAPH;
+}
 bool use_solo(const logo_ctx* c) {
-    return c->solo_ctas > 0 && c->descent_mode != LOGO_DESCENT_GRAPH &&
-           c->search == LOGO_SEARCH_EXHAUSTIVE;
+    return solo_runs(c) && c->search == LOGO_SEARCH_EXHAUSTIVE;
 }
 
 // Larger tours: the grid-wide launch, unless the caller asked for graphs or
 // chose the sweep kernel that descents are to run.
+bool grid_runs(const logo_ctx* c) {
+    return c->grid_ctas > 0 && c->descent_mode == LOGO_DESCENT_AUTO && !c->own_kernel;
+}
 bool use_grid(const logo_ctx* c) {
-    return c->grid_ctas > 0 && c->descent_mode == LOGO_DESCENT_AUTO && !c->own_kernel &&
-           c->search == LOGO_SEARCH_EXHAUSTIVE;
+    return grid_runs(c) && c->search == LOGO_SEARCH_EXHAUSTIVE;
+}
+
+// One launch runs the descent of the resident tour to its end: a cluster, or the
+// whole device.
+logo_status one_launch_descent(logo_ctx* c, uint32_t* route_out, bool* route_stored) {
+    std::unique_lock<std::mutex> lk;
+    if (solo_runs(c)) {
+        CK(c, launch_solo(solo_args(c), false, c->solo_ctas, c->stream));
+    } else {
+        lk = std::unique_lock<std::mutex>(coop_lock(c->device));
+        CK(c, launch_near_grid(grid_args(c), false, c->grid_ctas, c->stream));
+    }
+    logo_status s;
+    if (route_out) {
+        s = enqueue_route_out(c, route_out, false);
+        if (s != LOGO_OK) return s;
+        if (route_stored) *route_stored = true;
+    }
+    s = read_state(c);
+    if (s != LOGO_OK) return s;
+    if (!c->h_st->converged && !c->h_st->status)
+        return fail(c, LOGO_ERR_DEVICE_FAULT, "the descent did not finish");
+    return LOGO_OK;
 }
 
 // reset_enqueued: the reset was folded into the route load just before.
@@ -696,31 +723,14 @@ logo_status run_descent(logo_ctx* c, uint64_t max_moves, uint64_t* moves_out,
         sweeps0 = c->h_st->sweeps;
     }
     if (use_solo(c) || use_grid(c)) {
-        // one launch runs the whole descent: a cluster, or the whole device
-        std::unique_lock<std::mutex> lk;
-        if (use_solo(c)) {
-            CK(c, launch_solo(solo_args(c), false, c->solo_ctas, c->stream));
-        } else {
-            lk = std::unique_lock<std::mutex>(coop_lock(c->device));
-            CK(c, launch_near_grid(grid_args(c), false, c->grid_ctas, c->stream));
-        }
-        logo_status s;
-        if (route_out) {
-            s = enqueue_route_out(c, route_out, false);
-            if (s != LOGO_OK) return s;
-            if (route_stored) *route_stored = true;
-        }
-        s = read_state(c);
+        const logo_status s = one_launch_descent(c, route_out, route_stored);
         if (s != LOGO_OK) return s;
-        if (!c->h_st->converged && !c->h_st->status)
-            return fail(c, LOGO_ERR_DEVICE_FAULT, "the descent did not finish");
     } else if (c->search != LOGO_SEARCH_EXHAUSTIVE) {
         // neighbour sweeps until no candidate improves (one cooperative
         // launch where available), then full sweeps
         logo_status s;
         if (c->nbr_coop_grid > 0 && c->descent_mode != LOGO_DESCENT_GRAPH) {
-            CK(c, cudaMemsetAsync(c->d_coop, 0xFF, sizeof(CoopSync), c->stream));
-            CK(c, cudaMemsetAsync(c->d_coop, 0, 2 * sizeof(unsigned int), c->stream));
+            CK(c, cudaMemsetAsync(&c->d_coop->arrived, 0, sizeof(c->d_coop->arrived), c->stream));
             std::lock_guard<std::mutex> lk(coop_lock(c->device));
             CK(c, launch_coop_nbr(nbr_args(c), c->d_coop, c->nbr_coop_grid, c->stream));
             s = read_state(c);
@@ -730,8 +740,11 @@ logo_status run_descent(logo_ctx* c, uint64_t max_moves, uint64_t* moves_out,
         if (s != LOGO_OK) return s;
         if (!c->h_st->status && !c->h_st->bad_route) {
             CK(c, launch_resume_descent(bufs(c), c->stream));
-            s = graph_descent(c, max_moves, reset, moves0, c->h_st->moves, route_out,
-                              route_stored);
+            if (solo_runs(c) || grid_runs(c))
+                s = one_launch_descent(c, route_out, route_stored);
+            else
+                s = graph_descent(c, max_moves, reset, moves0, c->h_st->moves, route_out,
+                                  route_stored);
             if (s != LOGO_OK) return s;
         }
     } else {
@@ -1452,8 +1465,7 @@ logo_status logo_ils(logo_ctx* c, uint32_t* route, uint32_t kicks, uint64_t seed
         const bool nbr_coop = c->search != LOGO_SEARCH_EXHAUSTIVE && c->nbr_coop_grid > 0 &&
                               c->descent_mode != LOGO_DESCENT_GRAPH;
         if (nbr_coop) {  // the neighbour phases are cooperative kernel nodes
-            CK(c, cudaMemsetAsync(c->d_coop, 0xFF, sizeof(CoopSync), c->stream));
-            CK(c, cudaMemsetAsync(c->d_coop, 0, 2 * sizeof(unsigned int), c->stream));
+            CK(c, cudaMemsetAsync(&c->d_coop->arrived, 0, sizeof(c->d_coop->arrived), c->stream));
             std::lock_guard<std::mutex> lk(coop_lock(c->device));
             CK(c, cudaGraphLaunch(c->ils_exec, c->stream));
             s = read_state(c);

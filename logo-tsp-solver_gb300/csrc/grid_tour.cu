@@ -7,11 +7,8 @@
 // of a few dependent L2 reads and two grid barriers instead of four kernels that
 // go over windows, tiles and the whole tour (n = 100,000: 86 us a move).
 //
-// A grid barrier: each CTA leaves its best key, thread 0 adds to a counter
-// (release) and polls it (acquire, which also makes the SM's L1 current: the
-// arrays are read through it, and other SMs rewrite them between barriers;
-// bounded by %globaltimer, after which the CTA sets kErrTimeout and every CTA
-// gives up in turn).  Every CTA reads the same keys and so does the same.
+// Every CTA leaves its best key before a grid barrier (grid_barrier.cuh), reads the
+// same keys after it and so does the same.
 //
 // As a whole call the launch also loads and checks the caller's route and leaves
 // result and state in host memory: one launch and one wait (best move and move
@@ -26,6 +23,7 @@
 // slower (n = 20,000: 18.9 -> 20.8 us a sweep).
 #include <cstddef>
 
+#include "grid_barrier.cuh"
 #include "logo_device.cuh"
 #include "logo_internal.h"
 #include "near_tour.cuh"
@@ -38,44 +36,6 @@ constexpr int kGridNT = 1024;  // one CTA per SM
 constexpr unsigned long long kGridWaitNs = 20000000000ull;  // other kernels may hold SMs for long
 
 using GridTour = NearTour<uint32_t, kCtxNear>;
-
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-struct GridBarrier {
-    GridSync* gs;
-    DevState* st;
-    bool* ok;  // shared
-    unsigned long long target = 0;
-
-    // False when the wait ran out (the same in every thread of the CTA).
-    __device__ __forceinline__ bool operator()() {
-        target += gridDim.x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&gs->arrived) : "memory");
-            bool fine = true;
-            unsigned long long t0 = 0;
-            for (uint32_t it = 0; ld_acquire_u64(&gs->arrived) < target; ++it) {
-                if ((it & 255u) == 255u) {
-                    const unsigned long long now = global_timer_ns();
-                    if (t0 == 0) t0 = now;
-                    if (now - t0 > kGridWaitNs) {
-                        atomicOr(&st->status, kErrTimeout);
-                        fine = false;
-                        break;
-                    }
-                }
-            }
-            *ok = fine;
-        }
-        __syncthreads();
-        return *ok;
-    }
-};
 
 // Slot k = position k = city route[k], by all threads; a barrier must follow.
 __device__ __forceinline__ void grid_place(GridTour& T, const uint32_t* route, const float2* xy,
@@ -174,7 +134,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     T.cell = A.solo.near.cell;
     T.cellid = A.solo.near.cellid;
     T.g = A.solo.near.g;
-    GridBarrier barrier{A.gs, st, &bar_ok};
+    GridBarrier barrier{&A.gs->arrived, st, &bar_ok, kGridWaitNs};
     S.init();
     // this CTA's best key, and the counters of the next sweep
     uint32_t parity = 0;

@@ -119,8 +119,8 @@ cudaError_t launch_nbr_sweep(const NbrLaunch& L, cudaStream_t s);
 // Recomputes pos from the current tour.
 cudaError_t launch_fill_pos(const NbrLaunch& L, cudaStream_t s);
 // The whole neighbour phase of a descent as one cooperative launch
-// (coop.cu): moves until no candidate improves or st->max_moves; cs must
-// hold count = gen = 0 and every slot = kNoMove.  coop_nbr_grid: its CTAs
+// (coop.cu): moves until no candidate improves or st->max_moves; cs->arrived
+// must be 0 or what a launch of as many CTAs left.  coop_nbr_grid: its CTAs
 // for this n (0: cooperative launches unavailable).
 int coop_nbr_grid(uint32_t n, bool oropt, int device);
 cudaError_t launch_coop_nbr(const NbrLaunch& L, CoopSync* cs, int grid, cudaStream_t s);
@@ -228,11 +228,15 @@ int near_grid_ctas(uint32_t n, int device);
 cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t s);
 
 // State of a cooperative launch (coop.cu).
+// A CTA's best candidate of a sweep: its order (NbrPick in coop.cu), and the cities
+// of the list entry it came from.
+struct CoopBest {
+    unsigned long long lo;
+    uint32_t hi, city, near, pad;
+};
 struct CoopSync {
-    unsigned int count;            // CTAs arrived at the current barrier
-    unsigned int gen;              // barrier generation
-    unsigned long long slot[3];    // best key of move m in slot m % 3
-    unsigned long long or_slot[3][5];  // neighbour phase: Or-opt keys per variant
+    unsigned long long arrived;  // barrier arrivals so far; 0 before the first launch
+    CoopBest best[2][kGridMaxCtas];  // by the sweep's parity
 };
 // One CTA waits at the cooperative grid barrier sized for two (test hook).
 cudaError_t launch_barrier_probe(CoopSync* cs, DevState* st, cudaStream_t s);

@@ -9,31 +9,19 @@
 
 namespace logo {
 
-// Loads of the tour (ordered cities, route, positions).  kLdPlain: the
-// multi-kernel path, where the tour is read-only for the whole launch.
-// kLdCoherent: the cooperative phase, where other SMs rewrite the tour
-// between moves of one launch: coherent (ld.global.ca, never the read-only
-// path), made current after each grid barrier by its acquire.  kLdL2: the
-// same through L2 only.
-constexpr int kLdPlain = 0, kLdL2 = 1, kLdCoherent = 2;
-template <int LD>
+// Loads of the tour (ordered cities, route, positions) in the cooperative phase,
+// where other SMs rewrite it between moves of one launch: coherent (ld.global.ca,
+// never the read-only path), made current after each grid barrier by its acquire.
 __device__ __forceinline__ OrderedCity ld_city(const OrderedCity* p) {
-    if (LD != kLdPlain) {
-        const float4* q = reinterpret_cast<const float4*>(p);
-        const float4 v = LD == kLdL2 ? __ldcg(q) : __ldca(q);
-        OrderedCity o;
-        o.x = v.x;
-        o.y = v.y;
-        o.e = v.z;
-        o.pad = v.w;
-        return o;
-    }
-    return *p;
+    const float4 v = __ldca(reinterpret_cast<const float4*>(p));
+    OrderedCity o;
+    o.x = v.x;
+    o.y = v.y;
+    o.e = v.z;
+    o.pad = v.w;
+    return o;
 }
-template <int LD>
-__device__ __forceinline__ uint32_t ld_u32(const uint32_t* p) {
-    return LD == kLdPlain ? *p : (LD == kLdL2 ? __ldcg(p) : __ldca(p));
-}
+__device__ __forceinline__ uint32_t ld_u32(const uint32_t* p) { return __ldca(p); }
 
 constexpr uint32_t kNbrBatch = 4;  // neighbours whose loads are issued together
 
@@ -98,25 +86,25 @@ __device__ __forceinline__ void or_try(uint32_t s, uint32_t p, uint32_t n,
 // Every candidate of tour position i (its city's list: 2-opt pairs, and
 // with OR the Or-opt moves in which the city at i is a segment end); the
 // lowest 2-opt key goes to best and the lowest Or-opt key per variant to bo.
-template <bool OR, int LD = kLdPlain>
+template <bool OR>
 __device__ __forceinline__ void nbr_position(uint32_t i, const OrderedCity* __restrict__ Q,
                                              const uint32_t* __restrict__ R,
                                              const uint32_t* __restrict__ pos,
                                              const uint32_t* __restrict__ nbr, uint32_t K,
                                              uint32_t n, float M, uint64_t& best,
                                              uint64_t* bo) {
-    const uint32_t city = min(ld_u32<LD>(R + i), n - 1);
-    const OrderedCity qim = ld_city<LD>(Q + (i >= 1 ? i - 1 : 0)), qi = ld_city<LD>(Q + i),
-                      qip = ld_city<LD>(Q + min(i + 1, n - 1));
+    const uint32_t city = min(R[i], n - 1);
+    const OrderedCity qim = Q[i >= 1 ? i - 1 : 0], qi = Q[i],
+                      qip = Q[min(i + 1, n - 1)];
     // Or-opt: positions i-3 .. i+3 and the bases d(s-1, s+L) - e[s] - e[s+L]
     // of the segments (s, L) = (i, 1), (i, 2), (i, 3), (i-1, 2), (i-2, 3)
     OrderedCity qm3, qm2, qp2, qp3;
     int b1 = INT_MAX, b2 = INT_MAX, b3 = INT_MAX, c2 = INT_MAX, c3 = INT_MAX;
     if (OR) {
-        qm3 = ld_city<LD>(Q + (i >= 3 ? i - 3 : 0));
-        qm2 = ld_city<LD>(Q + (i >= 2 ? i - 2 : 0));
-        qp2 = ld_city<LD>(Q + min(i + 2, n - 1));
-        qp3 = ld_city<LD>(Q + min(i + 3, n - 1));
+        qm3 = Q[i >= 3 ? i - 3 : 0];
+        qm2 = Q[i >= 2 ? i - 2 : 0];
+        qp2 = Q[min(i + 2, n - 1)];
+        qp3 = Q[min(i + 3, n - 1)];
         if (i >= 1 && i + 1 <= n - 1)
             b1 = exact_dist(qim.x, qim.y, qip.x, qip.y) - (int)qi.e - (int)qip.e;
         if (i >= 1 && i + 2 <= n - 1)
@@ -134,13 +122,13 @@ __device__ __forceinline__ void nbr_position(uint32_t i, const OrderedCity* __re
 #pragma unroll
         for (uint32_t j = 0; j < kNbrBatch; ++j) p[j] = nb[min(k0 + j, K - 1)];
 #pragma unroll
-        for (uint32_t j = 0; j < kNbrBatch; ++j) p[j] = min(ld_u32<LD>(pos + min(p[j], n - 1)), n - 1);
+        for (uint32_t j = 0; j < kNbrBatch; ++j) p[j] = min(pos[min(p[j], n - 1)], n - 1);
         OrderedCity qpm[kNbrBatch], qp[kNbrBatch], qpp[kNbrBatch];
 #pragma unroll
         for (uint32_t j = 0; j < kNbrBatch; ++j) {
-            qpm[j] = ld_city<LD>(Q + (p[j] >= 1 ? p[j] - 1 : 0));
-            qp[j] = ld_city<LD>(Q + p[j]);
-            qpp[j] = ld_city<LD>(Q + min(p[j] + 1, n - 1));
+            qpm[j] = Q[p[j] >= 1 ? p[j] - 1 : 0];
+            qp[j] = Q[p[j]];
+            qpp[j] = Q[min(p[j] + 1, n - 1)];
         }
 #pragma unroll
         for (uint32_t j = 0; j < kNbrBatch; ++j) {

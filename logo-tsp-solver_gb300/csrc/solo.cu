@@ -211,10 +211,8 @@ __global__ void __launch_bounds__(NT) near_solo_kernel(SoloArgs A) {
             A.route_best[k] = id;
             A.Qbest[k] = OrderedCity{c.x, c.y, e, 0.f};
         }
-        if (whole) {
-            if (A.call.out) A.call.out[k] = id;
-            if (A.pos) A.pos[id] = k;
-        }
+        if (whole && A.call.out) A.call.out[k] = id;
+        if (A.pos) A.pos[id] = k;
     }
     unsigned long long end_len = 0;
     if (whole && A.call.lengths) end_len = near_length<NT>(T, S);

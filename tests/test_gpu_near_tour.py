@@ -142,3 +142,24 @@ def test_whole_calls_and_graph_agree(lg, inst, n):
                         st["final_length"], s.optimize_step(t), s.get_route()))
     for a, b in zip(*res):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "heaps", "clumps", "lattice"])
+@pytest.mark.parametrize("n", [8, 33, 1025, 6145, 80000])
+def test_neighbour_phase_and_graph_agree(lg, inst, n, kind):
+    """The neighbour phase as one launch against its kernels in a graph: from one
+    CTA to all, positions in more than one turn (80000), ties everywhere."""
+    xy = points(inst, kind, n, 90 + n)
+    r = lg.nn_tour(xy) if n > 2000 else inst.random_tour(n, 91 + n)
+    for search in (lg.SEARCH_NEIGHBOUR, lg.SEARCH_NEIGHBOUR_OROPT):
+        res = []
+        for mode in (lg.DESCENT_GRAPH, lg.DESCENT_AUTO):
+            with lg.Solver(xy) as s:
+                s.set_search(search)
+                s.set_descent_mode(mode)
+                t, st = s.optimize(r, max_moves=150 if n > 2000 else 0)
+                u, su = s.optimize(t, max_moves=20)
+            res.append((t, st["moves"], st["sweeps"], st["pair_evals"], u, su["moves"],
+                        su["sweeps"], su["final_length"]))
+        for a, b in zip(*res):
+            assert np.array_equal(a, b)
