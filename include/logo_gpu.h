@@ -466,12 +466,14 @@ logo_status logo_ctx_set_shape(logo_ctx *ctx, int rows_per_thread, int warps_per
                                uint32_t tile_cols);
 
 /* How a descent is driven; all modes return identical moves.
- * LOGO_DESCENT_AUTO (default): COOPERATIVE where available, else GRAPH.
+ * LOGO_DESCENT_AUTO (default): COOPERATIVE where available; larger tours as
+ *   one cooperative launch over the whole device (not after
+ *   logo_ctx_set_kernel or logo_ctx_set_shape); else GRAPH.
  * LOGO_DESCENT_GRAPH: captured CUDA graphs of (sweep, gather) launches,
  *   replayed until the device convergence flag is set.
- * LOGO_DESCENT_COOPERATIVE: one cooperative persistent launch per descent
+ * LOGO_DESCENT_COOPERATIVE: one launch of one thread-block cluster per descent
  *   (tours of 8 to 6,144 cities, held in every CTA's shared memory; one
- *   grid barrier per move).  No counterpart in the reference, whose descent is a
+ *   cluster barrier per move).  No counterpart in the reference, whose descent is a
  *   host loop over optimizeStep (src/solvers/twoOptLocalSolver.cpp:22-64). */
 #define LOGO_DESCENT_AUTO 0
 #define LOGO_DESCENT_GRAPH 1
@@ -510,7 +512,7 @@ logo_status logo_ctx_set_route_io(logo_ctx *ctx, int mode);
  *   at large n (no counterpart in the reference).  The neighbour phase of
  *   a descent is one cooperative launch where the device allows it (inside
  *   logo_ils a cooperative kernel node of its graph; graph launches with
- *   LOGO_DESCENT_GRAPH); the full sweeps after it use graph launches.
+ *   LOGO_DESCENT_GRAPH); the full sweeps after it run as without lists.
  * LOGO_SEARCH_NEIGHBOUR_OROPT: as NEIGHBOUR, and each step also weighs the
  *   Or-opt moves that create an edge to a listed neighbour: a segment of 1
  *   to 3 cities moved, in order or reversed, into another gap of the tour

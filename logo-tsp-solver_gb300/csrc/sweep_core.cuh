@@ -1,6 +1,6 @@
 // Per-thread core of the 2-opt sweep, shared by the single-instance kernel
-// (sweep.cu: one CTA per tile, columns staged by TMA) and the batched kernel
-// (batch.cu: whole instance in shared memory).
+// (sweep.cu: one CTA per tile, columns staged by TMA) and the dense tiles of
+// noalloc.cu.
 //
 // A thread owns pair rows ib .. ib+R-1 (and row ib-1 for the reuse) and walks
 // columns c upward.  With c = j + 1 (src/solvers/cpuSolver.cpp:188-230):

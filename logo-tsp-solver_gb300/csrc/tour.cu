@@ -6,9 +6,8 @@
 // the last CTA to finish (threadfence + counter, no spinning), so the host
 // never touches the tour between moves.  Where the context keeps city
 // positions (the boxed sweep's seed pass, the neighbour search), every
-// kernel that moves the tour writes them too; a position left stale (the
-// cooperative exhaustive descent does not write them) only weakens the
-// seed, never a result, because the seed pass evaluates whatever pair of
+// kernel that moves the tour writes them too; a position left stale would only
+// weaken the seed, never a result, because the seed pass evaluates whatever pair of
 // positions it reads exactly, and the neighbour search recomputes them
 // before its first use.
 //   load_route_kernel      ≙ ordered-coordinate gather, CUDASolver.cpp:316-319
