@@ -16,8 +16,8 @@
 // delta so far.  B is good before the sweep begins: every window's longest edge
 // is paired with every other's first.  The sweep is bound by the latency of its
 // four dependent launches then, not by the pairs (n = 20,011, clustered, NN tour:
-// 128 -> 55 us; a random tour 191 -> 38; a local optimum 128 -> 71; n = 65,536:
-// 810 -> 170, random 1,320 -> 160; n = 52: 29.5 -> 25.5).
+// 128 -> 58 us; a random tour 191 -> 41; a local optimum 128 -> 73; n = 65,536:
+// 810 -> 72, random 1,320 -> 62; n = 52: 29.5 -> 26.4).
 //
 // Its working memory (the tour-ordered cities, the argmin key, the bounding
 // box and a status word) lives in one file-scope __device__ array of fixed
@@ -238,12 +238,18 @@ constexpr int kCols = 4;  // columns whose loads are in flight together
 template <uint32_t COLS>
 constexpr uint32_t kWalkStepsOf = kRowWindows * COLS * 10 / 24;
 
-// grid (column chunk, row block); tiles entirely below the diagonal exit, and the
-// last of the `tiles` others leaves the result.
+// CTAs of the sweep at most, about two waves; above, each takes several column
+// chunks.  (Many CTAs cost more than their work, as they count themselves out on
+// one word: n = 65,536 with one chunk each 170 us; half as many CTAs leave too few
+// warps for long tiles, n = 20,011 at a local optimum 73 -> 86 us.)
+constexpr uint32_t kSweepCtas = 2736;
+
+// grid (group of `chunks` column chunks, row block); groups entirely below the
+// diagonal exit, and the last of the `tiles` others leaves the result.
 template <uint32_t kColWindows>
 __global__ void __launch_bounds__(kNW * 32)
-    noalloc_sweep(uint32_t n, uint32_t tiles, unsigned char* scratch, logo_move* out,
-                  int32_t* status_out) {
+    noalloc_sweep(uint32_t n, uint32_t chunks, uint32_t tiles, unsigned char* scratch,
+                  logo_move* out, int32_t* status_out) {
     constexpr uint32_t kColsPerCta = kColWindows * kWindow, kWalkSteps = kWalkStepsOf<kColsPerCta>;
     static_assert(kRowWindows * kColWindows <= 32, "a pair of windows per lane");
     chain_wait();
@@ -251,94 +257,98 @@ __global__ void __launch_bounds__(kNW * 32)
     const OrderedCity* Q = reinterpret_cast<const OrderedCity*>(scratch + sizeof(NoAllocHeader));
     __shared__ unsigned long long wbest[kNW];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t row0 = blockIdx.y * kRowsPerCta, col0 = blockIdx.x * kColsPerCta;
-    if (col0 + kColsPerCta <= row0) return;
+    const uint32_t row0 = blockIdx.y * kRowsPerCta, group = chunks * kColsPerCta;
+    if ((blockIdx.x + 1) * group <= row0) return;
     uint64_t best = kNoMove;
     if (!*(volatile unsigned int*)&h->status) {
         const float margin = h->margin;
         const unsigned long long known = *(volatile unsigned long long*)&h->key;
         int B = known == kNoMove ? -1 : key_delta(known);
         const uint32_t rows = row0 + warp * kRowsPerWarp;
-        // a lane per pair of windows
-        const uint32_t r0 = rows + lane / kColWindows * kWindow;
-        const uint32_t c0 = col0 + lane % kColWindows * kWindow;
-        float er = 0.f, ec = 0.f;  // their longest edges
-        bool hit = false;
-        if (lane < kRowWindows * kColWindows && r0 < n && c0 < n && c0 >= r0) {
-            const OrderedCity *R = Q + r0, *C = Q + c0;
-            er = R[kLongest].pad;
-            ec = C[kLongest].pad;
-            const float dx = fmaxf(fmaxf(C[kMinX].pad - R[kMaxX].pad, R[kMinX].pad - C[kMaxX].pad),
-                                   0.f);
-            const float dy = fmaxf(fmaxf(C[kMinY].pad - R[kMaxY].pad, R[kMinY].pad - C[kMaxY].pad),
-                                   0.f);
-            // (the two new edges, rounded, are no shorter than 2 d less 1 and the
-            // rounding of the differences, squares and roots)
-            const float d = sqrtf(dx * dx + dy * dy) * (1.f - 4e-6f);
-            hit = 2.f * d - 4.f <= er + ec + (float)B;
-        }
-        const uint32_t hits = __ballot_sync(0xffffffffu, hit);
-        uint32_t steps = 0;
-        if (__popc(hits) * kWindow > kWalkSteps) {
-            for (uint32_t t = 0; t < 32; ++t) {
-                if (!(hits >> t & 1u)) continue;
-                const uint32_t c = col0 + t % kColWindows * kWindow + lane;
-                const float e = __shfl_sync(0xffffffffu, er, t);
-                steps += __popc(__ballot_sync(
-                    0xffffffffu, c < n && Q[min(c, n - 1)].e + e + (float)B >= 0.f));
+        const uint32_t end = min((blockIdx.x + 1) * group, n);
+        for (uint32_t col0 = blockIdx.x * group; col0 < end; col0 += kColsPerCta) {
+            if (col0 + kColsPerCta <= rows) continue;
+            // a lane per pair of windows
+            const uint32_t r0 = rows + lane / kColWindows * kWindow;
+            const uint32_t c0 = col0 + lane % kColWindows * kWindow;
+            float er = 0.f, ec = 0.f;  // their longest edges
+            bool hit = false;
+            if (lane < kRowWindows * kColWindows && r0 < n && c0 < n && c0 >= r0) {
+                const OrderedCity *R = Q + r0, *C = Q + c0;
+                er = R[kLongest].pad;
+                ec = C[kLongest].pad;
+                const float dx = fmaxf(fmaxf(C[kMinX].pad - R[kMaxX].pad, R[kMinX].pad - C[kMaxX].pad),
+                                       0.f);
+                const float dy = fmaxf(fmaxf(C[kMinY].pad - R[kMaxY].pad, R[kMinY].pad - C[kMaxY].pad),
+                                       0.f);
+                // (the two new edges, rounded, are no shorter than 2 d less 1 and the
+                // rounding of the differences, squares and roots)
+                const float d = sqrtf(dx * dx + dy * dy) * (1.f - 4e-6f);
+                hit = 2.f * d - 4.f <= er + ec + (float)B;
             }
-        }
-        if (steps > kWalkSteps) {
-            const uint32_t ib = rows + lane * kR;
-            RowBlock<kR> rb;
-            load_rows<kR>(rb, Q, ib, n);
-            refresh_thresholds<kR>(rb, Q, ib, n, B, margin);
-            walk_columns<kR>(rb, Q, 0, col0, min(col0 + kColsPerCta, n), ib, n, Q, margin, B,
-                             best);
-        } else {
-            for (uint32_t g = 0; g < kRowWindows; ++g) {
-                uint32_t left = hits >> (g * kColWindows) & ((1u << kColWindows) - 1u);
-                if (left == 0) continue;
-                const uint32_t i = rows + g * kWindow + lane;
-                const bool row = i >= 1 && i + 3 <= n;
-                const OrderedCity q = Q[min(i, n - 1)], qm = Q[row ? i - 1 : 0];
-                const float longest =  // (any pair that is in has read it)
-                    __shfl_sync(0xffffffffu, er, g * kColWindows + __ffs(left) - 1);
-                for (; left; left &= left - 1) {
-                    const uint32_t w = __ffs(left) - 1;
-                    const float e = __shfl_sync(0xffffffffu, ec, g * kColWindows + w);
-                    if (!__any_sync(0xffffffffu, row && q.e + e + (float)B >= 0.f)) continue;
-                    const uint32_t first = col0 + w * kWindow, c = first + lane;
-                    uint32_t cols = __ballot_sync(
-                        0xffffffffu,
-                        c >= 1 && c < n && Q[min(c, n - 1)].e + longest + (float)B >= 0.f);
-                    while (cols) {  // kCols at a time, at the end the last one again
-                        uint32_t j[kCols];
-                        OrderedCity p[kCols], pm[kCols];
+            const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+            uint32_t steps = 0;
+            if (__popc(hits) * kWindow > kWalkSteps) {
+                for (uint32_t t = 0; t < 32; ++t) {
+                    if (!(hits >> t & 1u)) continue;
+                    const uint32_t c = col0 + t % kColWindows * kWindow + lane;
+                    const float e = __shfl_sync(0xffffffffu, er, t);
+                    steps += __popc(__ballot_sync(
+                        0xffffffffu, c < n && Q[min(c, n - 1)].e + e + (float)B >= 0.f));
+                }
+            }
+            if (steps > kWalkSteps) {
+                const uint32_t ib = rows + lane * kR;
+                RowBlock<kR> rb;
+                load_rows<kR>(rb, Q, ib, n);
+                refresh_thresholds<kR>(rb, Q, ib, n, B, margin);
+                walk_columns<kR>(rb, Q, 0, col0, min(col0 + kColsPerCta, n), ib, n, Q, margin, B,
+                                 best);
+            } else {
+                for (uint32_t g = 0; g < kRowWindows; ++g) {
+                    uint32_t left = hits >> (g * kColWindows) & ((1u << kColWindows) - 1u);
+                    if (left == 0) continue;
+                    const uint32_t i = rows + g * kWindow + lane;
+                    const bool row = i >= 1 && i + 3 <= n;
+                    const OrderedCity q = Q[min(i, n - 1)], qm = Q[row ? i - 1 : 0];
+                    const float longest =  // (any pair that is in has read it)
+                        __shfl_sync(0xffffffffu, er, g * kColWindows + __ffs(left) - 1);
+                    for (; left; left &= left - 1) {
+                        const uint32_t w = __ffs(left) - 1;
+                        const float e = __shfl_sync(0xffffffffu, ec, g * kColWindows + w);
+                        if (!__any_sync(0xffffffffu, row && q.e + e + (float)B >= 0.f)) continue;
+                        const uint32_t first = col0 + w * kWindow, c = first + lane;
+                        uint32_t cols = __ballot_sync(
+                            0xffffffffu,
+                            c >= 1 && c < n && Q[min(c, n - 1)].e + longest + (float)B >= 0.f);
+                        while (cols) {  // kCols at a time, at the end the last one again
+                            uint32_t j[kCols];
+                            OrderedCity p[kCols], pm[kCols];
 #pragma unroll
-                        for (int u = 0; u < kCols; ++u) {
-                            j[u] = cols ? first + __ffs(cols) - 1 : j[u ? u - 1 : 0];
-                            cols &= cols - 1;
-                            p[u] = Q[j[u]];
-                            pm[u] = Q[j[u] - 1];
-                        }
+                            for (int u = 0; u < kCols; ++u) {
+                                j[u] = cols ? first + __ffs(cols) - 1 : j[u ? u - 1 : 0];
+                                cols &= cols - 1;
+                                p[u] = Q[j[u]];
+                                pm[u] = Q[j[u] - 1];
+                            }
 #pragma unroll
-                        for (int u = 0; u < kCols; ++u) {
-                            const float v = approx_dist(q.x, q.y, p[u].x, p[u].y) +
-                                            (approx_dist(qm.x, qm.y, pm[u].x, pm[u].y) - p[u].e);
-                            if (row && j[u] >= i + 2 && v < (float)(B + (int)q.e) + margin) {
-                                const int delta = exact_dist(q.x, q.y, p[u].x, p[u].y) +
-                                                  exact_dist(qm.x, qm.y, pm[u].x, pm[u].y) -
-                                                  (int)q.e - (int)p[u].e;
-                                if (delta <= B) {
-                                    const uint64_t key = pack_key(delta, i, j[u]);
-                                    best = key < best ? key : best;
-                                    B = delta;
+                            for (int u = 0; u < kCols; ++u) {
+                                const float v = approx_dist(q.x, q.y, p[u].x, p[u].y) +
+                                                (approx_dist(qm.x, qm.y, pm[u].x, pm[u].y) - p[u].e);
+                                if (row && j[u] >= i + 2 && v < (float)(B + (int)q.e) + margin) {
+                                    const int delta = exact_dist(q.x, q.y, p[u].x, p[u].y) +
+                                                      exact_dist(qm.x, qm.y, pm[u].x, pm[u].y) -
+                                                      (int)q.e - (int)p[u].e;
+                                    if (delta <= B) {
+                                        const uint64_t key = pack_key(delta, i, j[u]);
+                                        best = key < best ? key : best;
+                                        B = delta;
+                                    }
                                 }
                             }
                         }
+                        B = __reduce_min_sync(0xffffffffu, B);
                     }
-                    B = __reduce_min_sync(0xffffffffu, B);
                 }
             }
         }
@@ -436,9 +446,15 @@ extern "C" logo_status logo_best_move_noalloc(const logo_xy* coords, const uint3
     unsigned char* sc = static_cast<unsigned char*>(scratch);
     const bool few = n <= kFewMax;
     const uint32_t cols = (few ? kColWindowsFew : kColWindowsMost) * kWindow;
-    const dim3 grid((n + cols - 1) / cols, (n + kRowsPerCta - 1) / kRowsPerCta);
-    uint32_t tiles = 0;
-    for (uint32_t y = 0; y < grid.y; ++y) tiles += grid.x - y * (kRowsPerCta / cols);
+    const uint32_t rows = (n + kRowsPerCta - 1) / kRowsPerCta;
+    uint32_t chunks = 1, tiles = 0;
+    dim3 grid;
+    for (;; chunks *= 2) {
+        grid = dim3((n + cols * chunks - 1) / (cols * chunks), rows);
+        tiles = 0;
+        for (uint32_t y = 0; y < rows; ++y) tiles += grid.x - y * kRowsPerCta / (cols * chunks);
+        if (tiles <= kSweepCtas) break;
+    }
     const float2* xy = reinterpret_cast<const float2*>(coords);
     const uint32_t groups = ((n + kWindow - 1) / kWindow + 31) / 32;
     constexpr uint32_t kPairs = kSeedThreads / 32;
@@ -448,7 +464,7 @@ extern "C" logo_status logo_best_move_noalloc(const logo_xy* coords, const uint3
         launch_chained(noalloc_seed, (groups * groups + kPairs - 1) / kPairs, kSeedThreads, 0, s,
                        n, sc) != cudaSuccess ||
         launch_chained(few ? noalloc_sweep<kColWindowsFew> : noalloc_sweep<kColWindowsMost>, grid,
-                       kNW * 32, 0, s, n, tiles, sc, out, status_out) != cudaSuccess)
+                       kNW * 32, 0, s, n, chunks, tiles, sc, out, status_out) != cudaSuccess)
         return LOGO_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? LOGO_OK : LOGO_ERR_CUDA;
 }
