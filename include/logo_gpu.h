@@ -591,6 +591,14 @@ logo_status logo_diag_wait_limits(int device, uint32_t *mbarrier_status,
  * (a context whose device wait timed out is never used again; destroy it). */
 logo_status logo_diag_flag_timeout(logo_ctx *ctx);
 
+/* Test hooks of the grid-wide launch (tours above 6,144 cities): how many edges
+ * put off in a sweep it lists, how many edges it lists for their pairs, and from
+ * how many cities a disc is put off (0: the library's own limits, which are also
+ * the largest); results never depend on them.  The counts are the largest of any
+ * sweep of the context's last such launch. */
+logo_status logo_diag_grid_limits(logo_ctx *ctx, uint32_t wide, uint32_t takers, uint32_t disc);
+logo_status logo_diag_grid_counts(logo_ctx *ctx, uint32_t *wide, uint32_t *takers);
+
 /* Self-check of the sweep's exactness argument: the largest relative error of
  * the device's approximate square root over every positive normal binary32
  * input, against the correctly rounded root.  The sweep's filter margin

@@ -60,6 +60,7 @@ struct logo_ctx {
     int solo_ils_ctas = 0;        // the same for a whole ILS call
     int grid_ctas = 0;            // CTAs of the grid-wide descent of larger tours (0: unavailable)
     GridSync* d_grid = nullptr;
+    uint32_t grid_wide = kGridWide, grid_takers = kGridTakers, grid_disc = kGridDisc;
     bool own_kernel = false;      // the caller chose a sweep kernel: descents run that one
     int descent_mode = LOGO_DESCENT_AUTO;
     uint2* d_tiles = nullptr;
@@ -191,6 +192,9 @@ GridArgs grid_args(const logo_ctx* c) {
     GridArgs A{};
     A.solo = solo_args(c);
     A.gs = c->d_grid;
+    A.wide = c->grid_wide;
+    A.takers = c->grid_takers;
+    A.disc = c->grid_disc;
     return A;
 }
 
@@ -1208,6 +1212,29 @@ logo_status logo_diag_flag_timeout(logo_ctx* c) {
     CK(c, cudaMemcpyAsync(&c->d_st->status, &bit, sizeof(bit), cudaMemcpyHostToDevice,
                           c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
+    return LOGO_OK;
+}
+
+logo_status logo_diag_grid_limits(logo_ctx* c, uint32_t wide, uint32_t takers, uint32_t disc) {
+    if (!c) return LOGO_ERR_INVALID_ARG;
+    if (wide > kGridWide || takers > kGridTakers || disc > kGridDisc)
+        return fail(c, LOGO_ERR_INVALID_ARG, "above the library's own limits");
+    c->grid_wide = wide ? wide : kGridWide;
+    c->grid_takers = takers ? takers : kGridTakers;
+    c->grid_disc = disc ? disc : kGridDisc;
+    return LOGO_OK;
+}
+
+logo_status logo_diag_grid_counts(logo_ctx* c, uint32_t* wide, uint32_t* takers) {
+    if (!c || !wide || !takers) return LOGO_ERR_INVALID_ARG;
+    if (!c->d_grid) return fail(c, LOGO_ERR_INVALID_ARG, "no grid-wide launches at this size");
+    CK(c, cudaSetDevice(c->device));
+    uint32_t most[2] = {0u, 0u};
+    CK(c, cudaMemcpyAsync(most, &c->d_grid->most_wides, sizeof(most), cudaMemcpyDeviceToHost,
+                          c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
+    *wide = most[0];
+    *takers = most[1];
     return LOGO_OK;
 }
 

@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     unsigned long long m = 0, sweeps = 0, total_m = 0;
     unsigned long long best_len = 0, accepted = 0, kicks = 0;
     uint64_t rng = 0;
+    uint32_t most_wides = 0, most_takers = 0;
     if (ILS) {
         best_len = *(volatile unsigned long long*)&st->best_length;
         rng = *(volatile unsigned long long*)&st->rng;
@@ -195,13 +196,14 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     for (uint32_t it = 0; ok; ++it) {
         m = 0;
         for (;;) {
-            NearBest nb{near_scan<NT, false>(T, S, seed, parity, rank, ranks), -1.f};
+            NearBest nb{near_scan<NT, false>(T, S, seed, parity, rank, ranks, A.disc), -1.f};
             const uint32_t z = T.closing();
             __syncthreads();
             const uint32_t huges = S.huges[parity];  // the same for every thread
             if (huges) {
                 // the edges of these slots that reach beyond their lists
-                if (nb.key != kNoMove) nb.B = (float)key_delta(nb.key);
+                // (the CTA's bound, not the lane's own best: near_far wants one for the warp)
+                nb.B = fminf((float)S.bound[parity], (float)S.far_bound[parity]);
                 const float h = near_half((float)S.bound[parity]);
                 for (uint32_t o = warp; o < 2 * huges; o += NW) {
                     const uint32_t j = S.huge[o / 2], f = o & 1 ? T.wrap(j + 1) : j;
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
                     uint32_t at = 0;
                     if (lane == 0) at = atomicAdd(&A.gs->wides[parity], 1u);
                     at = __shfl_sync(0xffffffffu, at, 0);
-                    if (at >= kGridWide)
+                    if (at >= A.wide)
                         near_far(T, j, z, ~0u, nb.B, nb);  // no room for this one
                     else if (lane == 0)
                         A.gs->wide[parity][at] = f;
@@ -232,7 +234,8 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             }
             __syncthreads();
             uint64_t key = best_key;
-            const uint32_t wides = min(wide_count, kGridWide);
+            const uint32_t wides = min(wide_count, A.wide);
+            most_wides = max(most_wides, wide_count);
             if (wides) {
                 // edges put off, with every edge that can take part: listed first,
                 // so that the pairs can be dealt evenly, unless those are too many
@@ -245,11 +248,12 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
                     uint32_t at = 0;
                     if (lane == 0) at = atomicAdd(&A.gs->takers[parity], (uint32_t)__popc(votes));
                     at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1u));
-                    if (takes && at < kGridTakers) A.gs->taker[at] = g;
+                    if (takes && at < A.takers) A.gs->taker[at] = g;
                 }
                 if (!(ok = barrier())) break;
                 const uint32_t takers = *(volatile uint32_t*)&A.gs->takers[parity];
-                if (takers <= kGridTakers) {
+                most_takers = max(most_takers, takers);
+                if (takers <= A.takers) {
                     for (uint32_t base = tid - lane; base < wides * takers; base += threads) {
                         const uint32_t t = base + lane;
                         const bool in = t < wides * takers;
@@ -380,6 +384,8 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             if (bad) atomicOr(&st->status, kErrBadKey);
         }
         st->converged = step && ok ? 0u : 1u;
+        A.gs->most_wides = most_wides;
+        A.gs->most_takers = most_takers;
     }
     if (whole) leave();
 }

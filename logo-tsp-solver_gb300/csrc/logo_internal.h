@@ -204,6 +204,7 @@ cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s);
 // whole device (grid_tour.cu): one CTA per SM.
 constexpr uint32_t kGridMaxCtas = 256;
 constexpr uint32_t kGridWide = 1024, kGridTakers = 8192;
+constexpr uint32_t kGridDisc = 4096;  // cities of a disc that one CTA goes through
 struct GridSync {
     unsigned long long arrived;    // barrier arrivals so far
     unsigned long long length[2];  // tour length of the descent in hand, by its parity
@@ -218,10 +219,13 @@ struct GridSync {
     uint32_t wide[2][kGridWide];
     uint32_t taker[kGridTakers];
     unsigned long long keys[2][kGridMaxCtas];  // best key per CTA, by the sweep's parity
+    uint32_t most_wides, most_takers;  // largest counts of a sweep of the last launch
 };
 struct GridArgs {
     SoloArgs solo;  // pos: slot of every city meanwhile
     GridSync* gs;
+    // limits, at most (a test's are smaller) kGridWide, kGridTakers and kGridDisc
+    uint32_t wide, takers, disc;
 };
 // CTAs of the launch (0: n is not above kSoloMaxN, or not available).
 int near_grid_ctas(uint32_t n, int device);

@@ -152,7 +152,6 @@ struct NearTour {
 constexpr uint32_t kNearFar = 256;   // discs of a sweep's CTA that may wait for their warps
 constexpr uint32_t kNearWide = 64;   // discs that may be put off again, to the whole CTA
 constexpr uint32_t kNearDisc = 256;  // cities that a warp goes through of a disc
-constexpr uint32_t kGridDisc = 4096;  // and a CTA, where many CTAs share a tour in global memory
 
 // MAXC: CTAs that share the sweeps (a cluster, each with its own copy of the tour).
 template <int NT, int MAXC, typename IX>
@@ -579,8 +578,9 @@ __device__ __forceinline__ bool near_meet(const TOUR& T, bool in, uint32_t j, ui
 // A slot whose list was too short, looked at by the whole warp: the grid's
 // cells in the disc that bound B gives, of whose cities this warp takes part
 // `part` of `parts` (B has to be the same in all of those warps: they number the
-// disc's cities alike).  j is the slot (the same in every lane).  A disc of more
-// than `most` cities is left alone, and the result is true.
+// disc's cities alike).  j, most, B and nb.B are the same in every lane: the warp
+// goes through the cells together.  A disc of more than `most` cities is left
+// alone, and the result is true.
 template <typename TOUR>
 __device__ __forceinline__ bool near_far(const TOUR& T, uint32_t j, uint32_t z,
                                          uint32_t most, float B, NearBest& nb,
@@ -779,12 +779,13 @@ __device__ __forceinline__ uint32_t near_lists(const TOUR& T, SLOTS& w, uint32_t
 //    until every list has been looked at because a disc costs what its radius
 //    says and the radius shrinks with the bound, which the CTA's warps share.
 // 4. Large discs are put off to all warps of the CTA, which take a part each
-//    (those beyond kGridDisc stay in S.huge for the caller), or with ALL_EDGES go
+//    (those beyond `huge` stay in S.huge for the caller), or with ALL_EDGES go
 //    over the edges that can take part instead (long edges of a tour far from a
 //    local optimum: the bound is large then, and most edges too short).
 template <int NT, bool ALL_EDGES, typename TOUR, typename SH>
 __device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSeed& seed,
-                                              uint32_t parity, uint32_t rank, uint32_t ranks) {
+                                              uint32_t parity, uint32_t rank, uint32_t ranks,
+                                              uint32_t huge = ~0u) {
     using IX = typename TOUR::Index;
     constexpr int NW = NT / 32;
     const uint32_t n = T.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -893,7 +894,7 @@ __device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSe
     if (!ALL_EDGES) {
         // (alike in all warps: the size depends on `bound` alone)
         for (uint32_t o = 0; o < big; ++o)
-            if (near_far(T, S.wide[o], z, kGridDisc, bound, nb, warp, NW) && threadIdx.x == 0)
+            if (near_far(T, S.wide[o], z, huge, bound, nb, warp, NW) && threadIdx.x == 0)
                 S.huge[S.huges[parity]++] = S.wide[o];
     } else if (big) {
         for (uint32_t base = warp * 32; base < n; base += NT) {  // whole warps

@@ -58,7 +58,7 @@ EXPORTS = [
     "logo_server_create", "logo_server_submit", "logo_server_poll", "logo_server_wait",
     "logo_server_get_stats", "logo_server_destroy", "logo_server_last_error",
     "logo_diag_flag_timeout", "logo_ctx_set_route_io", "logo_ctx_set_search",
-    "logo_neighbours", "logo_start_tour",
+    "logo_neighbours", "logo_start_tour", "logo_diag_grid_limits", "logo_diag_grid_counts",
 ]
 
 
@@ -192,6 +192,8 @@ def load(path=LIB_PATH):
                                      c.c_uint64, c.POINTER(Stats)]
     L.logo_diag_sqrt_error.argtypes = [c.c_int, ctypes.POINTER(ctypes.c_double)]
     L.logo_diag_flag_timeout.argtypes = [_vp]
+    L.logo_diag_grid_limits.argtypes = [_vp, c.c_uint32, c.c_uint32, c.c_uint32]
+    L.logo_diag_grid_counts.argtypes = [_vp, _u32p, _u32p]
     L.logo_diag_wait_limits.argtypes = [c.c_int, ctypes.POINTER(ctypes.c_uint32),
                                         ctypes.POINTER(ctypes.c_uint32),
                                         ctypes.POINTER(ctypes.c_double)]
@@ -426,6 +428,17 @@ class Solver:
         """Test hook: marks the context's device status as a timed-out wait
         would (logo_diag_flag_timeout)."""
         _check(load().logo_diag_flag_timeout(self._h), self._h)
+
+    def grid_limits(self, wide=0, takers=0, disc=0):
+        """Test hook: limits of the grid-wide launch (logo_diag_grid_limits)."""
+        _check(load().logo_diag_grid_limits(self._h, wide, takers, disc), self._h)
+
+    def grid_counts(self):
+        """Test hook: most edges put off and most edges listed for them in a
+        sweep of the last grid-wide launch (logo_diag_grid_counts)."""
+        a, b = ctypes.c_uint32(), ctypes.c_uint32()
+        _check(load().logo_diag_grid_counts(self._h, ctypes.byref(a), ctypes.byref(b)), self._h)
+        return a.value, b.value
 
 
 def read_tsplib(path):
