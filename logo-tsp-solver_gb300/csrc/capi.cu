@@ -299,16 +299,17 @@ logo_status rebuild(logo_ctx* c) {
         // positions are written by every kernel that moves the tour; until a
         // route is uploaded they only need to be in range
         CK(c, cudaMalloc(&c->d_pos, sizeof(uint32_t) * c->n));
-        CK(c, cudaMemset(c->d_pos, 0, sizeof(uint32_t) * c->n));
+        CK(c, cudaMemsetAsync(c->d_pos, 0, sizeof(uint32_t) * c->n, c->stream));
     }
     std::vector<uint2> tiles = make_tiles(c->n, c->R, c->NW, c->cb);
     c->ntiles = (uint32_t)tiles.size();
     if (c->ntiles) {
         CK(c, cudaMalloc(&c->d_work, sizeof(uint4) * tiles.size()));
         CK(c, cudaMalloc(&c->d_tiles, sizeof(uint2) * tiles.size()));
-        CK(c, cudaMemcpy(c->d_tiles, tiles.data(), sizeof(uint2) * tiles.size(),
-                         cudaMemcpyHostToDevice));
+        CK(c, cudaMemcpyAsync(c->d_tiles, tiles.data(), sizeof(uint2) * tiles.size(),
+                              cudaMemcpyHostToDevice, c->stream));
     }
+    CK(c, cudaStreamSynchronize(c->stream));  // the copies have left host memory
     // the sweep's shared-memory opt-in must be set outside stream capture
     CK(c, launch_sweep_prepare(sweep_args(c)));
     c->chunk_steps = pick_graph_steps(c->n);
@@ -363,21 +364,24 @@ logo_status prepare_search(logo_ctx* c) {
         CK(c, cudaMalloc(&c->d_coop, sizeof(CoopSync)));
     if (!c->d_pos) {
         CK(c, cudaMalloc(&c->d_pos, sizeof(uint32_t) * c->n));
-        CK(c, cudaMemset(c->d_pos, 0, sizeof(uint32_t) * c->n));
+        CK(c, cudaMemsetAsync(c->d_pos, 0, sizeof(uint32_t) * c->n, c->stream));
     }
     if (c->have_route)  // positions were not kept while nothing needed them
         CK(c, launch_fill_pos(nbr_args(c), c->stream));
     if (c->nbr_list_k != c->search_k) {
         std::vector<logo_xy> h(c->n);
-        CK(c, cudaMemcpy(h.data(), c->d_xy, sizeof(logo_xy) * c->n, cudaMemcpyDeviceToHost));
+        CK(c, cudaMemcpyAsync(h.data(), c->d_xy, sizeof(logo_xy) * c->n, cudaMemcpyDeviceToHost,
+                              c->stream));
+        CK(c, cudaStreamSynchronize(c->stream));
         std::vector<uint32_t> nb((size_t)c->n * c->search_k);
         knn_grid(h.data(), c->n, c->search_k, nb.data());
         if (c->d_nbr_search) cudaFree(c->d_nbr_search);
         c->d_nbr_search = nullptr;
         c->nbr_list_k = 0;
         CK(c, cudaMalloc(&c->d_nbr_search, sizeof(uint32_t) * nb.size()));
-        CK(c, cudaMemcpy(c->d_nbr_search, nb.data(), sizeof(uint32_t) * nb.size(),
-                         cudaMemcpyHostToDevice));
+        CK(c, cudaMemcpyAsync(c->d_nbr_search, nb.data(), sizeof(uint32_t) * nb.size(),
+                              cudaMemcpyHostToDevice, c->stream));
+        CK(c, cudaStreamSynchronize(c->stream));
         c->nbr_list_k = c->search_k;
     }
     CK(c, cudaStreamSynchronize(c->stream));
@@ -988,7 +992,10 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     CKC(cudaMalloc(&c->d_st, sizeof(DevState)));
     CKC(cudaMallocHost(&c->h_st, sizeof(DevState)));
     CKC(cudaMalloc(&c->d_seen, sizeof(uint32_t) * n));
-    CKC(cudaMemset(c->d_seen, 0, sizeof(uint32_t) * n));
+    // copies and clears go to the context's own stream: it is not ordered with the
+    // default stream, on which a copy from pageable memory may still be under way
+    // when the call returns
+    CKC(cudaMemsetAsync(c->d_seen, 0, sizeof(uint32_t) * n, c->stream));
     {
         int pageable = 0;
         if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) !=
@@ -1006,21 +1013,21 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     std::memset(c->h_st, 0, sizeof(DevState));
     c->h_st->best_key = kNoMove;
     c->h_st->converged = 1;
-    CKC(cudaMemcpy(c->d_st, c->h_st, sizeof(DevState), cudaMemcpyHostToDevice));
-    CKC(cudaMemcpy(c->d_xy, coords, sizeof(float2) * n, cudaMemcpyHostToDevice));
+    CKC(cudaMemcpyAsync(c->d_st, c->h_st, sizeof(DevState), cudaMemcpyHostToDevice, c->stream));
+    CKC(cudaMemcpyAsync(c->d_xy, coords, sizeof(float2) * n, cudaMemcpyHostToDevice, c->stream));
     c->grid_ctas = near_grid_ctas(n, device);
     if (c->grid_ctas > 0) {
         CKC(cudaMalloc(&c->d_grid, sizeof(GridSync)));
         CKC(cudaMalloc(&c->d_pos, sizeof(uint32_t) * n));
-        CKC(cudaMemset(c->d_pos, 0, sizeof(uint32_t) * n));
+        CKC(cudaMemsetAsync(c->d_pos, 0, sizeof(uint32_t) * n, c->stream));
     }
     CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n)));
     near_index_carve(c->near, c->d_near, n);
     c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
-    CKC(launch_near_index(c->near, c->d_xy, n, c->stream));
-#undef CKC
     s = rebuild(c);
     if (s != LOGO_OK) return bail(s);
+    CKC(launch_near_index(c->near, c->d_xy, n, c->stream));
+#undef CKC
     *out = c;
     return LOGO_OK;
 }
