@@ -503,7 +503,10 @@ __device__ __forceinline__ void cluster_store(uint32_t* p, uint32_t cta, uint32_
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(p)), "r"(cta));
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
 }
+// (the aligned form wants whole warps: a loop or branch before it may have left the
+// warp's threads apart)
 __device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                      : "memory");
 }
@@ -962,7 +965,6 @@ __device__ __forceinline__ uint64_t near_sweep(const TOUR& T, SH& S, NearSeed& s
     }
     if (threadIdx.x == 0) S.reset(parity ^ 1);  // the next sweep's
     if constexpr (CL) {
-        __syncwarp();
         cluster_barrier();
     } else {
         __syncthreads();
