@@ -529,8 +529,6 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
     batch_kernel(BatchArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ NearShared<NT, 1, uint16_t> S;
-    uint32_t parity = 0;
-    S.init();
 
     for (;;) {
         if (threadIdx.x == 0) S.idx = atomicAdd(A.queue, 1u);
@@ -545,6 +543,8 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
         uint32_t* rio = A.routes + I.off;
         CtaTour T = near_carve(smem_raw, n);
         NearSeed seed;
+        uint32_t parity = 0;
+        S.init();  // (the last instance's sweeps need not have left it so)
 
         // load (or build) the start tour; rio holds the best tour from here on
         if (A.start == kStartNN) {  // the list area holds the builder's two arrays

@@ -186,7 +186,8 @@ struct NearShared {
         bound[parity] = far_bound[parity] = -1;
         fars[parity] = big[parity] = huges[parity] = 0;
     }
-    // once per kernel; a barrier must follow before the first sweep
+    // once per instance, between barriers: sweeps (parity from 0) leave the counters of
+    // one parity as they are
     __device__ __forceinline__ void init() {
         if (threadIdx.x < 2) reset(threadIdx.x);
     }

@@ -36,8 +36,6 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
     serve_round_kernel(ServeArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ NearShared<NT, 1, uint16_t> S;
-    uint32_t parity = 0;
-    S.init();
 
     for (;;) {
         if (threadIdx.x == 0) S.idx = atomicAdd(A.queue, 1u);
@@ -54,6 +52,8 @@ __global__ void __launch_bounds__(NT, kNearWarpsPerSm * 32 / NT)
         uint32_t* bio = A.best + st.off;
         CtaTour T = near_carve(smem_raw, n);
         NearSeed seed;
+        uint32_t parity = 0;
+        S.init();  // (the last slot's sweeps need not have left it so)
 
         // load the resident tour into shared memory (the best one stays in the arena)
         for (uint32_t k = threadIdx.x; k < n; k += NT) {
