@@ -34,6 +34,8 @@ struct logo_ctx {
     uint32_t* d_route_best = nullptr;
     DevState* d_st = nullptr;
     DevState* h_st = nullptr;  // pinned mirror
+    unsigned long long* h_crowd = nullptr;  // behind it: see launch_near_index
+    mutable bool crowd_known = false;       // (once the lists are built)
     uint32_t* d_seen = nullptr;   // route permutation check: last load that met each city
     uint32_t load_epoch = 0;      // loads so far (mod 2^32 - 1, from 1)
     int route_io = LOGO_ROUTE_IO_AUTO;
@@ -207,6 +209,30 @@ uint64_t pair_evals_of(const logo_ctx* c, uint64_t sweeps, uint64_t nbr) {
     nbr = std::min(nbr, sweeps);
     const uint64_t per = (c->search == LOGO_SEARCH_NEIGHBOUR_OROPT ? 12ull : 2ull) * c->search_k;
     return (sweeps - nbr) * pairs_of(c->n) + nbr * per * c->n;
+}
+
+// Where the search grid's cells lie: the cities' box less what few cities far from
+// the rest stretch it by (twice the range of all but 1/64 of a sample of them at
+// either end holds every city of evenly spread instances).  Cities outside belong
+// to the outermost cells; the grid's users only need cells in the cities' order.
+// (One stray city at a hundred times the others' range, n = 100,000: without this
+// nearly all cities are in four cells and a sweep takes 1,216 us; with it 53.)
+void search_box(const logo_xy* xy, uint32_t n, double& x0, double& y0, double& x1, double& y1) {
+    constexpr uint32_t kSample = 1024, kEnd = kSample / 64;
+    if (n < kSample) return;
+    std::vector<double> v(kSample);
+    auto trim = [&](bool y, double& lo, double& hi) {
+        for (uint32_t k = 0; k < kSample; ++k) {
+            const logo_xy& p = xy[(uint64_t)k * n / kSample];
+            v[k] = y ? p.y : p.x;
+        }
+        std::sort(v.begin(), v.end());
+        const double a = v[kEnd], b = v[kSample - 1 - kEnd], more = 0.5 * (b - a);
+        lo = std::max(lo, a - more);
+        hi = std::min(hi, b + more);
+    };
+    trim(false, x0, x1);
+    trim(true, y0, y1);
 }
 
 // Default tile shape by size (overridable through logo_ctx_set_shape and
@@ -677,9 +703,27 @@ bool use_solo(const logo_ctx* c) {
 }
 
 // Larger tours: the grid-wide launch, unless the caller asked for graphs or
-// chose the sweep kernel that descents are to run.
+// chose the sweep kernel that descents are to run, or the search grid does not
+// tell the cities apart (a few dense heaps far from one another): each disc then
+// costs the cities of whole cells, while the sweeps over windows of the tour do not
+// care.  Measured (us a sweep of the first 400 moves of an NN tour, graphs and the
+// grid-wide launch, with the sum over all cities of the cities in their cell):
+// n = 20,000 in 2 heaps, 1.3e8: 96, 156; in 10, 3.8e7: 65, 44; 20 clusters, 8e6:
+// 57, 35; n = 100,000 in 2 heaps, 5e9: 247, 3,814; in 10, 9.5e8: 127, 1,597; in 50,
+// 2e8: 94, 99; in 200, 4.9e7: 90, 64; 20 clusters, 6.7e7: 81, 72; uniform, 3.5e5:
+// 75, 49.  A graph's sweep grows with the tour above that size (372 us at n = 1,000,000)
+// and the line with it.
+unsigned long long crowd_most(uint32_t n) { return std::max(100000000ull, 500ull * n); }
+bool crowded(const logo_ctx* c) {
+    if (!c->crowd_known) {
+        if (cudaStreamSynchronize(c->stream) != cudaSuccess) return false;  // (the call says so)
+        c->crowd_known = true;
+    }
+    return *c->h_crowd > crowd_most(c->n);
+}
 bool grid_runs(const logo_ctx* c) {
-    return c->grid_ctas > 0 && c->descent_mode == LOGO_DESCENT_AUTO && !c->own_kernel;
+    return c->grid_ctas > 0 && c->descent_mode == LOGO_DESCENT_AUTO && !c->own_kernel &&
+           !crowded(c);
 }
 bool use_grid(const logo_ctx* c) {
     return grid_runs(c) && c->search == LOGO_SEARCH_EXHAUSTIVE;
@@ -990,7 +1034,8 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     CKC(cudaMalloc(&c->d_Qbest, sizeof(OrderedCity) * n));
     CKC(cudaMalloc(&c->d_route_best, sizeof(uint32_t) * n));
     CKC(cudaMalloc(&c->d_st, sizeof(DevState)));
-    CKC(cudaMallocHost(&c->h_st, sizeof(DevState)));
+    CKC(cudaMallocHost(&c->h_st, sizeof(DevState) + sizeof(unsigned long long)));
+    c->h_crowd = reinterpret_cast<unsigned long long*>(c->h_st + 1);
     CKC(cudaMalloc(&c->d_seen, sizeof(uint32_t) * n));
     // copies and clears go to the context's own stream: it is not ordered with the
     // default stream, on which a copy from pageable memory may still be under way
@@ -1023,10 +1068,11 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     }
     CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n)));
     near_index_carve(c->near, c->d_near, n);
+    search_box(coords, n, x0, y0, x1, y1);
     c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
     s = rebuild(c);
     if (s != LOGO_OK) return bail(s);
-    CKC(launch_near_index(c->near, c->d_xy, n, c->stream));
+    CKC(launch_near_index(c->near, c->d_xy, n, c->h_crowd, c->stream));
 #undef CKC
     *out = c;
     return LOGO_OK;

@@ -156,7 +156,9 @@ struct NearIndex {
 // 32-bit words behind nbr, cell, cellid and seeds.
 size_t near_index_words(uint32_t n);
 void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);  // words 8-byte aligned
-cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s);
+// *crowd (pinned host memory): over all cities, the cities of its cell, summed.
+cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n,
+                              unsigned long long* crowd, cudaStream_t s);
 
 // A whole call as one launch: the route is loaded (and checked) by the launch
 // itself, and its state and result are left in host memory.

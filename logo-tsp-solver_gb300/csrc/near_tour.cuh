@@ -583,8 +583,10 @@ __device__ __forceinline__ bool near_meet(const TOUR& T, bool in, uint32_t j, ui
 // cells in the disc that bound B gives, of whose cities this warp takes part
 // `part` of `parts` (B has to be the same in all of those warps: they number the
 // disc's cities alike).  j, most, B and nb.B are the same in every lane: the warp
-// goes through the cells together.  A disc of more than `most` cities is left
-// alone, and the result is true.
+// goes through the cells together.  A disc of more than `most` cities, or of as many
+// cells as hold `most` on average, is left alone, and the result is true.  (The
+// cities are counted: where a few cities far from the rest stretch the box, one
+// cell may hold nearly all of them.)
 template <typename TOUR>
 __device__ __forceinline__ bool near_far(const TOUR& T, uint32_t j, uint32_t z,
                                          uint32_t most, float B, NearBest& nb,
@@ -599,14 +601,24 @@ __device__ __forceinline__ bool near_far(const TOUR& T, uint32_t j, uint32_t z,
     const int xa = near_cell(ux - r, T.g.inv, T.g.gx), xb = near_cell(ux + r, T.g.inv, T.g.gx);
     const int ya = near_cell(uy - r, T.g.inv, T.g.gy), yb = near_cell(uy + r, T.g.inv, T.g.gy);
     if (2u * (uint32_t)((xb - xa + 1) * (yb - ya + 1)) > most) return true;
-    for (int y0 = ya; y0 <= yb; y0 += 32) {
-        // up to 32 rows of cells, one per lane: each a run of cellid
-        const int y = y0 + (int)lane;
-        uint32_t first = 0, len = 0;
+    // up to 32 rows of cells, one per lane: each a run of cellid
+    uint32_t first = 0, len = 0;
+    auto row_of = [&](int y) {
+        first = len = 0;
         if (y <= yb) {
             first = T.cell[y * T.g.gx + xa];
             len = T.cell[y * T.g.gx + xb + 1] - first;
         }
+    };
+    row_of(ya + (int)lane);
+    if (most != ~0u) {
+        uint32_t held = len;
+        for (int y = ya + 32 + (int)lane; y <= yb; y += 32)
+            held += T.cell[y * T.g.gx + xb + 1] - T.cell[y * T.g.gx + xa];
+        if (__reduce_add_sync(0xffffffffu, held) > most) return true;
+    }
+    for (int y0 = ya; y0 <= yb; y0 += 32) {
+        if (y0 != ya) row_of(y0 + (int)lane);
         uint32_t end = len;
         for (int s = 1; s < 32; s <<= 1) {
             const uint32_t u = __shfl_up_sync(0xffffffffu, end, s);

@@ -254,15 +254,20 @@ __global__ void near_count_kernel(const float2* __restrict__ xy, uint32_t n, Nea
 }
 
 // Exclusive scan of count[0 .. cells) into cell[0 .. cells] and back into
-// count, by one CTA of 1,024 threads.
+// count, by one CTA of 1,024 threads; *crowd (host memory) gets the sum of the
+// squared counts.
 __global__ void __launch_bounds__(1024) near_scan_kernel(uint32_t* count, uint32_t* cell,
-                                                         uint32_t cells) {
+                                                         uint32_t cells,
+                                                         unsigned long long* crowd) {
     __shared__ uint32_t part[32];
+    __shared__ unsigned long long squares[32];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t carry = 0;
+    unsigned long long mine = 0;
     for (uint32_t base = 0; base < cells; base += 1024) {
         const uint32_t c = base + threadIdx.x;
         const uint32_t own = c < cells ? count[c] : 0u;
+        mine += (unsigned long long)own * own;
         uint32_t run = own;
         for (int s = 1; s < 32; s <<= 1) {
             const uint32_t u = __shfl_up_sync(0xffffffffu, run, s);
@@ -280,7 +285,14 @@ __global__ void __launch_bounds__(1024) near_scan_kernel(uint32_t* count, uint32
         carry += all;
         __syncthreads();
     }
-    if (threadIdx.x == 0) cell[cells] = carry;
+    mine = warp_sum_u64(mine);
+    if (lane == 0) squares[warp] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cell[cells] = carry;
+        for (uint32_t w = 1; w < 32; ++w) mine += squares[w];
+        *(volatile unsigned long long*)crowd = mine;
+    }
 }
 
 __global__ void near_scatter_kernel(const float2* __restrict__ xy, uint32_t n, NearGrid g,
@@ -380,14 +392,15 @@ void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n) {
     I.seeds = I.cellid + n;
 }
 
-cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n, cudaStream_t s) {
+cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n,
+                              unsigned long long* crowd, cudaStream_t s) {
     const uint32_t cells = (uint32_t)I.g.gx * (uint32_t)I.g.gy;
     const uint32_t grid = (n + 255) / 256;
     uint32_t* count = reinterpret_cast<uint32_t*>(I.nbr);
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t) * cells, s);
     if (e != cudaSuccess) return e;
     near_count_kernel<<<grid, 256, 0, s>>>(xy, n, I.g, count);
-    near_scan_kernel<<<1, 1024, 0, s>>>(count, I.cell, cells);
+    near_scan_kernel<<<1, 1024, 0, s>>>(count, I.cell, cells, crowd);
     near_scatter_kernel<<<grid, 256, 0, s>>>(xy, n, I.g, count, I.cellid);
     near_lists_kernel<<<(n + 127) / 128, 128, 0, s>>>(xy, n, I);
     return cudaGetLastError();

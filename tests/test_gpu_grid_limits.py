@@ -38,3 +38,44 @@ def test_limits_above_the_lists_are_refused(lg, inst):
         for limits in ((1025, 0, 0), (0, 8193, 0), (0, 0, 4097)):
             with pytest.raises(lg.LogoError):
                 s.grid_limits(*limits)
+
+
+def both_ways(lg, xy, r, moves, limits=(0, 0, 0)):
+    res = []
+    for mode in (lg.DESCENT_GRAPH, lg.DESCENT_AUTO):
+        with lg.Solver(xy) as s:
+            s.set_descent_mode(mode)
+            s.grid_limits(*limits)
+            t, trace, st = s.optimize_trace(r, max_moves=moves)
+            counts = s.grid_counts() if len(xy) > 6144 else None
+            res.append((t, trace, st["sweeps"], st["final_length"], s.optimize_step(t)))
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
+    return counts
+
+
+def test_a_disc_is_counted_by_its_cities(lg, inst):
+    """Two heaps far apart: each lies in one cell of the search grid, so a disc
+    of one cell holds thousands of cities and has to be put off."""
+    xy = inst.uniform_f32(7000, 11, 100.0)
+    xy[::2] += np.float32(1.0e6)
+    assert both_ways(lg, xy, lg.nn_tour(xy), 120, limits=(0, 0, 1024))[0] > 0
+
+
+@pytest.mark.parametrize("kind", ["stray", "strays", "heaps"])
+@pytest.mark.parametrize("n", [1024, 6000, 7000, 20000, 60000])
+def test_unevenly_spread_cities(lg, inst, n, kind):
+    """Cities far from the rest, which lie outside the search grid's box, and
+    heaps that its cells do not tell apart (from 20000 the graph-driven descent
+    runs there whatever the mode)."""
+    xy = inst.uniform_f32(n, 11 + n, 1.0e4)
+    if kind == "stray":
+        xy[n // 3] = (1.0e6, 1.0e6)
+    elif kind == "strays":
+        xy[7::n // 20] *= np.float32(-90.0)
+    else:
+        xy *= np.float32(0.01)
+        xy[::2] += np.float32(1.0e6)
+    both_ways(lg, xy, lg.nn_tour(xy), 100)
+    if n <= 20000:
+        both_ways(lg, xy, inst.random_tour(n, n), 60)
