@@ -598,6 +598,10 @@ logo_status logo_diag_flag_timeout(logo_ctx *ctx);
  * sweep of the context's last such launch. */
 logo_status logo_diag_grid_limits(logo_ctx *ctx, uint32_t wide, uint32_t takers, uint32_t disc);
 logo_status logo_diag_grid_counts(logo_ctx *ctx, uint32_t *wide, uint32_t *takers);
+/* Test hook: after how many microseconds a grid-wide launch ends between two moves
+ * to let other work onto the device (0: the default, 20000); results never depend on
+ * it. */
+logo_status logo_diag_grid_quantum(logo_ctx *ctx, uint32_t us);
 
 /* Self-check of the sweep's exactness argument: the largest relative error of
  * the device's approximate square root over every positive normal binary32

@@ -10,6 +10,7 @@
 // reads one small status block per replay.
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -63,6 +64,7 @@ struct logo_ctx {
     int grid_ctas = 0;            // CTAs of the grid-wide descent of larger tours (0: unavailable)
     GridSync* d_grid = nullptr;
     uint32_t grid_wide = kGridWide, grid_takers = kGridTakers, grid_disc = kGridDisc;
+    unsigned long long grid_quantum_ns = kGridQuantumNs;
     bool own_kernel = false;      // the caller chose a sweep kernel: descents run that one
     int descent_mode = LOGO_DESCENT_AUTO;
     uint2* d_tiles = nullptr;
@@ -197,6 +199,7 @@ GridArgs grid_args(const logo_ctx* c) {
     A.wide = c->grid_wide;
     A.takers = c->grid_takers;
     A.disc = c->grid_disc;
+    A.quantum_ns = c->grid_quantum_ns;
     return A;
 }
 
@@ -614,7 +617,31 @@ logo_status poisoned_error(logo_ctx* c) {
 logo_status status_to_error(logo_ctx* c, unsigned int st);
 bool use_solo(const logo_ctx* c);
 bool use_grid(const logo_ctx* c);
-std::mutex& coop_lock(int device);
+class TurnLock;
+TurnLock& coop_lock(int device);
+logo_status one_launch_descent(logo_ctx* c, uint32_t* route_out, bool* route_stored);
+
+// A lock that is handed on in the order in which it was asked for.
+class TurnLock {
+public:
+    void lock() {
+        std::unique_lock<std::mutex> lk(mu_);
+        const uint64_t mine = next_++;
+        cv_.wait(lk, [&] { return turn_ == mine; });
+    }
+    void unlock() {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            ++turn_;
+        }
+        cv_.notify_all();
+    }
+
+private:
+    std::mutex mu_;
+    std::condition_variable cv_;
+    uint64_t next_ = 0, turn_ = 0;
+};
 
 // A descent of the caller's route, or with step one sweep of it, as one launch
 // (the context's use_solo or use_grid holds): the launch loads and checks the
@@ -643,7 +670,7 @@ logo_status whole_call(logo_ctx* c, const uint32_t* route, uint32_t* out,
     call.step = step;
     call.lengths = lengths;
     c->have_route = false;
-    std::unique_lock<std::mutex> lk;
+    std::unique_lock<TurnLock> lk;
     if (use_solo(c)) {
         SoloArgs A = solo_args(c);
         A.call = call;
@@ -651,14 +678,24 @@ logo_status whole_call(logo_ctx* c, const uint32_t* route, uint32_t* out,
     } else {
         GridArgs A = grid_args(c);
         A.solo.call = call;
-        lk = std::unique_lock<std::mutex>(coop_lock(c->device));
+        lk = std::unique_lock<TurnLock>(coop_lock(c->device));
         CK(c, launch_near_grid(A, false, c->grid_ctas, c->stream));
     }
     ++c->host_waits;
     CK(c, cudaStreamSynchronize(c->stream));
+    if (lk.owns_lock()) lk.unlock();
     if (c->h_st->bad_route)
         return fail(c, LOGO_ERR_INVALID_ARG, "route is not a permutation of 0..n-1");
     c->have_route = true;
+    if (!step && !c->h_st->converged && !c->h_st->status) {  // paused: the descent goes on
+        if (stored) *stored = false;
+        logo_status s = one_launch_descent(c, nullptr, nullptr);
+        if (s == LOGO_OK && lengths && !(c->h_st->status & ~kErrMoveLimit)) {
+            CK(c, launch_tour_length(bufs(c), c->stream));
+            s = read_state(c);
+        }
+        if (s != LOGO_OK) return s;
+    }
     const unsigned int st = c->h_st->status & ~kErrMoveLimit;
     if (st) return status_to_error(c, st);
     return LOGO_OK;
@@ -686,12 +723,12 @@ logo_status graph_descent(logo_ctx* c, uint64_t max_moves, bool partial_ok, uint
                           bool nbr = false);
 logo_status enqueue_route_out(logo_ctx* c, uint32_t* route, bool best);
 
-// Cooperative descents of this library never overlap on one device: each
-// grid is sized to be resident on its own, and two whose CTAs were only
-// partly resident would wait on each other's SMs until their barriers gave
-// up.  The lock is held from the launch to its completion.
-std::mutex& coop_lock(int device) {
-    static std::mutex locks[64];
+// Cooperative launches of this library never overlap on one device (each is sized
+// to be resident on its own).  The lock is held from a launch to its completion, and
+// contexts take turns: a grid-wide descent gives it up with every launch that
+// pauses.
+TurnLock& coop_lock(int device) {
+    static TurnLock locks[64];
     return locks[(unsigned)device % 64];
 }
 
@@ -729,23 +766,36 @@ bool use_grid(const logo_ctx* c) {
     return grid_runs(c) && c->search == LOGO_SEARCH_EXHAUSTIVE;
 }
 
-// One launch runs the descent of the resident tour to its end: a cluster, or the
-// whole device.
+// A grid-wide launch of this context, ILS or descent, waited for with its turn on the
+// device; then the next while they pause.
+logo_status run_grid(logo_ctx* c, const GridArgs& A, bool ils) {
+    for (unsigned long long before = ~0ull;;) {
+        std::unique_lock<TurnLock> lk(coop_lock(c->device));
+        CK(c, launch_near_grid(A, ils, c->grid_ctas, c->stream));
+        const logo_status s = read_state(c);
+        if (s != LOGO_OK || c->h_st->converged || c->h_st->status) return s;
+        // a launch pauses after a move
+        if (c->h_st->total_moves == before)
+            return fail(c, LOGO_ERR_DEVICE_FAULT, "descent made no progress");
+        before = c->h_st->total_moves;
+    }
+}
+
+// The descent of the resident tour to its end: one launch of a cluster, or launches
+// over the whole device.
 logo_status one_launch_descent(logo_ctx* c, uint32_t* route_out, bool* route_stored) {
-    std::unique_lock<std::mutex> lk;
+    logo_status s;
     if (solo_runs(c)) {
         CK(c, launch_solo(solo_args(c), false, c->solo_ctas, c->stream));
+        if (route_out) {
+            s = enqueue_route_out(c, route_out, false);
+            if (s != LOGO_OK) return s;
+            if (route_stored) *route_stored = true;
+        }
+        s = read_state(c);
     } else {
-        lk = std::unique_lock<std::mutex>(coop_lock(c->device));
-        CK(c, launch_near_grid(grid_args(c), false, c->grid_ctas, c->stream));
+        s = run_grid(c, grid_args(c), false);
     }
-    logo_status s;
-    if (route_out) {
-        s = enqueue_route_out(c, route_out, false);
-        if (s != LOGO_OK) return s;
-        if (route_stored) *route_stored = true;
-    }
-    s = read_state(c);
     if (s != LOGO_OK) return s;
     if (!c->h_st->converged && !c->h_st->status)
         return fail(c, LOGO_ERR_DEVICE_FAULT, "the descent did not finish");
@@ -783,7 +833,7 @@ logo_status run_descent(logo_ctx* c, uint64_t max_moves, uint64_t* moves_out,
         logo_status s;
         if (c->nbr_coop_grid > 0 && c->descent_mode != LOGO_DESCENT_GRAPH) {
             CK(c, cudaMemsetAsync(&c->d_coop->arrived, 0, sizeof(c->d_coop->arrived), c->stream));
-            std::lock_guard<std::mutex> lk(coop_lock(c->device));
+            std::lock_guard<TurnLock> lk(coop_lock(c->device));
             CK(c, launch_coop_nbr(nbr_args(c), c->d_coop, c->nbr_coop_grid, c->stream));
             s = read_state(c);
         } else {
@@ -1291,6 +1341,12 @@ logo_status logo_diag_grid_counts(logo_ctx* c, uint32_t* wide, uint32_t* takers)
     return LOGO_OK;
 }
 
+logo_status logo_diag_grid_quantum(logo_ctx* c, uint32_t us) {
+    if (!c) return LOGO_ERR_INVALID_ARG;
+    c->grid_quantum_ns = us ? 1000ull * us : kGridQuantumNs;
+    return LOGO_OK;
+}
+
 logo_status logo_set_route(logo_ctx* c, const uint32_t* route) {
     if (!c) return LOGO_ERR_INVALID_ARG;
     if (c->poisoned) return poisoned_error(c);
@@ -1537,16 +1593,14 @@ logo_status logo_ils(logo_ctx* c, uint32_t* route, uint32_t kicks, uint64_t seed
         GridArgs A = grid_args(c);
         A.solo.kicks = kicks;
         A.solo.kick_kind = kick_kind;
-        std::lock_guard<std::mutex> lk(coop_lock(c->device));
-        CK(c, launch_near_grid(A, true, c->grid_ctas, c->stream));
-        s = read_state(c);
+        s = run_grid(c, A, true);
     } else {
         // one graph: descent and kick loops are WHILE nodes on device conditions
         const bool nbr_coop = c->search != LOGO_SEARCH_EXHAUSTIVE && c->nbr_coop_grid > 0 &&
                               c->descent_mode != LOGO_DESCENT_GRAPH;
         if (nbr_coop) {  // the neighbour phases are cooperative kernel nodes
             CK(c, cudaMemsetAsync(&c->d_coop->arrived, 0, sizeof(c->d_coop->arrived), c->stream));
-            std::lock_guard<std::mutex> lk(coop_lock(c->device));
+            std::lock_guard<TurnLock> lk(coop_lock(c->device));
             CK(c, cudaGraphLaunch(c->ils_exec, c->stream));
             s = read_state(c);
         } else {

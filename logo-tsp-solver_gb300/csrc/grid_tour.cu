@@ -10,6 +10,10 @@
 // Every CTA leaves its best key before a grid barrier (grid_barrier.cuh), reads the
 // same keys after it and so does the same.
 //
+// The launch holds every SM (a CTA's registers are all that an SM has), so nothing
+// else runs beside it: after quantum_ns it ends, between two moves, with everything
+// in the state, and the host launches it again behind whatever else is waiting.
+//
 // As a whole call the launch also loads and checks the caller's route and leaves
 // result and state in host memory: one launch and one wait (best move and move
 // of a 100,000-city route: 111 -> 60 us; best move of 1,000,000: 612 -> 168 us,
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     __shared__ bool bar_ok;
     __shared__ uint2 seeds[32];
     __shared__ unsigned long long best_key;
-    __shared__ uint32_t wide_count;
+    __shared__ uint32_t wide_count, pause_now;
     DevState* st = A.solo.st;
     const bool whole = !ILS && A.solo.call.src != nullptr;
     // set before the launch and identical for every CTA
@@ -117,6 +121,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     const uint32_t n = A.solo.n, rank = blockIdx.x, ranks = gridDim.x;
     const uint32_t tid = rank * NT + threadIdx.x, threads = ranks * NT;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned long long begun = tid == 0 ? global_timer_ns() : 0ull;
     const uint32_t cur = whole ? 0u : *(volatile unsigned int*)&st->cur;
     OrderedCity* Qg = cur ? A.solo.Q1 : A.solo.Q0;
     uint32_t* Rg = cur ? A.solo.R1 : A.solo.R0;
@@ -192,8 +197,8 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
         best_len = *(volatile unsigned long long*)&st->best_length;
         rng = *(volatile unsigned long long*)&st->rng;
     }
-    bool limit = false, bad = false;
-    for (uint32_t it = 0; ok; ++it) {
+    bool limit = false, bad = false, paused = false;
+    for (uint32_t it = ILS ? (uint32_t)*(volatile unsigned long long*)&st->kicks : 0u; ok; ++it) {
         m = 0;
         for (;;) {
             NearBest nb{near_scan<NT, false>(T, S, seed, parity, rank, ranks, A.disc), -1.f};
@@ -217,6 +222,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
                         A.gs->wide[parity][at] = f;
                 }
             }
+            if (tid == 0) A.gs->pause[parity] = global_timer_ns() - begun > A.quantum_ns;
             publish(A.gs->keys[parity], nb.key);
             if (!(ok = barrier())) break;
             ++sweeps;
@@ -225,11 +231,13 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             // lines queued up at L2 for 7 us)
             if (warp == 0) {
                 const uint32_t w = *(volatile uint32_t*)&A.gs->wides[parity];
+                const uint32_t pause = *(volatile uint32_t*)&A.gs->pause[parity];
                 const uint64_t k = near_pick(T, A.gs->keys[parity], ranks, seed);
                 seeds[lane] = make_uint2(seed.a, seed.b);
                 if (lane == 0) {
                     best_key = k;
                     wide_count = w;
+                    pause_now = pause;
                 }
             }
             __syncthreads();
@@ -303,9 +311,13 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
                 limit = true;
                 break;
             }
+            if (pause_now) {  // (the same in every CTA)
+                paused = true;
+                break;
+            }
         }
         total_m += m;
-        if (!ILS || !ok || bad) break;
+        if (!ILS || !ok || bad || paused) break;
         // length of the tour; keep it if strictly shorter than the best, else go back
         unsigned long long part = 0;
         for (uint32_t k = tid; k < n; k += threads) part += (unsigned long long)T.E[k];
@@ -355,10 +367,10 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             Rg[k] = id;
             Qg[k] = o;
             T.pos[id] = k;
-            if (ILS) A.solo.Qbest[k] = o;
-            if (whole && A.solo.call.out) A.solo.call.out[k] = id;
+            if (ILS && !paused) A.solo.Qbest[k] = o;
+            if (whole && A.solo.call.out && !paused) A.solo.call.out[k] = id;
         }
-        if (lengths) {
+        if (lengths && !paused) {
             part = warp_sum_u64(part);
             if (lane == 0 && part) atomicAdd(&A.gs->length[0], part);
             ok = barrier();
@@ -366,7 +378,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     }
     if (lengths && tid == 0) {
         st->start_length = ld_acquire_u64(&A.gs->start_length);
-        st->length = ld_acquire_u64(&A.gs->length[0]);
+        if (!paused) st->length = ld_acquire_u64(&A.gs->length[0]);
     }
     if (tid == 0) {
         if (ok) {
@@ -383,7 +395,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             if (limit) atomicOr(&st->status, kErrMoveLimit);
             if (bad) atomicOr(&st->status, kErrBadKey);
         }
-        st->converged = step && ok ? 0u : 1u;
+        st->converged = (step || paused) && ok ? 0u : 1u;
         A.gs->most_wides = most_wides;
         A.gs->most_takers = most_takers;
     }

@@ -216,6 +216,7 @@ struct GridSync {
     // by its parity (more may have been offered than fit)
     uint32_t wides[2], takers[2];
     uint32_t left;  // CTAs that have left a whole call
+    uint32_t pause[2];  // the launch is to end after this sweep's move, by its parity
     // (set to zero up to here before a launch)
     unsigned long long wide_keys[2][kGridMaxCtas];  // best key per CTA after those
     uint32_t wide[2][kGridWide];
@@ -228,8 +229,16 @@ struct GridArgs {
     GridSync* gs;
     // limits, at most (a test's are smaller) kGridWide, kGridTakers and kGridDisc
     uint32_t wide, takers, disc;
+    unsigned long long quantum_ns;  // a launch that has run for longer ends after its next move
 };
-// CTAs of the launch (0: n is not above kSoloMaxN, or not available).
+// Default of quantum_ns: how long other work on the device (another context's call, a
+// serving round) waits for one launch.  Going on costs a launch, the tour's way into
+// the ring and back, and a first sweep without the last one's seeds (every 2 ms 6 %, every
+// 20 ms 0.2 % of an ILS call at n = 20,000).
+constexpr unsigned long long kGridQuantumNs = 20000000ull;
+// CTAs of the launch (0: n is not above kSoloMaxN, or not available).  The state it
+// leaves is not converged when it paused: the next launch goes on from it (of an ILS
+// call in the middle of a descent, after st->kicks kicks).
 int near_grid_ctas(uint32_t n, int device);
 cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t s);
 

@@ -59,6 +59,7 @@ EXPORTS = [
     "logo_server_get_stats", "logo_server_destroy", "logo_server_last_error",
     "logo_diag_flag_timeout", "logo_ctx_set_route_io", "logo_ctx_set_search",
     "logo_neighbours", "logo_start_tour", "logo_diag_grid_limits", "logo_diag_grid_counts",
+    "logo_diag_grid_quantum",
 ]
 
 
@@ -194,6 +195,7 @@ def load(path=LIB_PATH):
     L.logo_diag_flag_timeout.argtypes = [_vp]
     L.logo_diag_grid_limits.argtypes = [_vp, c.c_uint32, c.c_uint32, c.c_uint32]
     L.logo_diag_grid_counts.argtypes = [_vp, _u32p, _u32p]
+    L.logo_diag_grid_quantum.argtypes = [_vp, c.c_uint32]
     L.logo_diag_wait_limits.argtypes = [c.c_int, ctypes.POINTER(ctypes.c_uint32),
                                         ctypes.POINTER(ctypes.c_uint32),
                                         ctypes.POINTER(ctypes.c_double)]
@@ -432,6 +434,10 @@ class Solver:
     def grid_limits(self, wide=0, takers=0, disc=0):
         """Test hook: limits of the grid-wide launch (logo_diag_grid_limits)."""
         _check(load().logo_diag_grid_limits(self._h, wide, takers, disc), self._h)
+
+    def grid_quantum(self, us=0):
+        """Test hook: when a grid-wide launch pauses (logo_diag_grid_quantum)."""
+        _check(load().logo_diag_grid_quantum(self._h, us), self._h)
 
     def grid_counts(self):
         """Test hook: most edges put off and most edges listed for them in a
