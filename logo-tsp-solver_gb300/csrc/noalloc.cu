@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(kSeedThreads) noalloc_seed(uint32_t n, unsigne
         const double dx = (double)from_ordered(h->bbox[2]) - (double)from_ordered(h->bbox[0]);
         const double dy = (double)from_ordered(h->bbox[3]) - (double)from_ordered(h->bbox[1]);
         const double diag = sqrt(dx * dx + dy * dy);
-        if (!(diag < LOGO_MAX_DIAGONAL)) atomicExch(&h->status, (unsigned int)LOGO_ERR_INVALID_ARG);
+        if (n >= 4 && !(diag < LOGO_MAX_DIAGONAL))  // (three cities have no move, at any distance)
+            atomicExch(&h->status, (unsigned int)LOGO_ERR_INVALID_ARG);
         h->margin = noalloc_margin(diag);
     }
     if (row > col || row >= groups) return;  // whole warps
