@@ -451,11 +451,13 @@ typedef struct logo_ctx_info {
     int descent_mode;     /* LOGO_DESCENT_* in use */
     int cooperative_ctas; /* CTAs of the cooperative descent; 0 if unavailable */
     uint64_t host_waits;  /* times this context's calls have waited on the device so far
-                             (one logo_ils call: a fixed handful, whatever the kick count) */
+                             (one logo_ils call: a fixed handful, whatever the kick count;
+                             as grid-wide launches one more for every 20 ms) */
     int route_io;         /* LOGO_ROUTE_IO_COPY or LOGO_ROUTE_IO_DIRECT in use */
     int search;           /* LOGO_SEARCH_* */
     uint32_t search_neighbours; /* neighbour-list length of LOGO_SEARCH_NEIGHBOUR */
-    uint32_t pad0;
+    uint32_t grid_ctas;   /* CTAs of the grid-wide launch, which has the whole device to itself,
+                             that descents and ILS calls run as; 0 if they do not */
 } logo_ctx_info;
 
 logo_status logo_ctx_get_info(const logo_ctx *ctx, logo_ctx_info *info);

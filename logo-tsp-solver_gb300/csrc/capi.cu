@@ -1150,7 +1150,7 @@ logo_status logo_ctx_get_info(const logo_ctx* c, logo_ctx_info* info) {
     info->route_io = route_direct(c) ? LOGO_ROUTE_IO_DIRECT : LOGO_ROUTE_IO_COPY;
     info->search = c->search;
     info->search_neighbours = c->search_k;
-    info->pad0 = 0;
+    info->grid_ctas = grid_runs(c) ? (uint32_t)c->grid_ctas : 0u;
     return LOGO_OK;
 }
 

@@ -93,7 +93,7 @@ class CtxInfo(ctypes.Structure):
                 ("variant", ctypes.c_int), ("descent_mode", ctypes.c_int),
                 ("cooperative_ctas", ctypes.c_int), ("host_waits", ctypes.c_uint64),
                 ("route_io", ctypes.c_int), ("search", ctypes.c_int),
-                ("search_neighbours", ctypes.c_uint32), ("pad0", ctypes.c_uint32)]
+                ("search_neighbours", ctypes.c_uint32), ("grid_ctas", ctypes.c_uint32)]
 
 
 class Instance(ctypes.Structure):

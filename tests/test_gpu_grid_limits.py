@@ -79,3 +79,21 @@ def test_unevenly_spread_cities(lg, inst, n, kind):
     both_ways(lg, xy, lg.nn_tour(xy), 100)
     if n <= 20000:
         both_ways(lg, xy, inst.random_tour(n, n), 60)
+
+
+def test_info_says_when_calls_run_over_the_whole_device(lg, inst):
+    xy = inst.uniform_f32(20000, 1, 1.0e4)
+    with lg.Solver(xy[:6144]) as s:
+        assert s.info()["grid_ctas"] == 0
+    with lg.Solver(xy) as s:
+        assert s.info()["grid_ctas"] > 0
+        s.set_descent_mode(lg.DESCENT_GRAPH)
+        assert s.info()["grid_ctas"] == 0
+        s.set_descent_mode(lg.DESCENT_AUTO)
+        assert s.info()["grid_ctas"] > 0
+        s.set_kernel(lg.SWEEP_BOXED, 4, 4, 64)
+        assert s.info()["grid_ctas"] == 0
+    heaps = xy * np.float32(0.01)
+    heaps[::2] += np.float32(1.0e6)
+    with lg.Solver(heaps) as s:  # its search grid would not tell the cities apart
+        assert s.info()["grid_ctas"] == 0
