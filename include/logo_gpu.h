@@ -311,7 +311,9 @@ typedef struct logo_server_opts {
     uint32_t max_large;     /* larger requests in flight; 0 = 2 */
     uint32_t kicks;         /* ILS kicks per request after its first descent */
     int kick_kind;          /* LOGO_KICK_* */
-    uint64_t quantum_pairs; /* pair evaluations per request per round; 0 = 2e7 */
+    uint64_t quantum_pairs; /* work per request and round, in pair evaluations, of which a
+                               sweep counts as 16 a city (what its lists hold); 0 = 2e7; a
+                               quarter of it while a request above 6,144 cities runs */
     uint32_t max_pending;   /* submitted but not admitted; 0 = 1,000,000 */
 } logo_server_opts;
 

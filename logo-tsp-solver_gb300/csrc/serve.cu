@@ -28,7 +28,9 @@ namespace {
 
 // Pair evaluations charged per city and sweep: a sweep looks at a few listed
 // neighbours of each city (near_tour.cuh counts them), 16 is what its lists
-// hold.
+// hold.  (The default quantum is then 305 sweeps at n = 4,096, a round of 23 ms of
+// which 2 go into the lists of clustered cities, built anew in every round; charged
+// 48, rounds of 11 ms and a burst of 64 requests up to 15 % slower.)
 constexpr unsigned long long kServePairsPerCity = 16;
 
 template <int NT>
