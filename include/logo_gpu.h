@@ -90,7 +90,9 @@ typedef struct logo_ctx logo_ctx;
 /* ---- single instance ------------------------------------------------------ */
 
 /* Creates a context for one instance on `device` and copies the coordinates
- * to it.  Replaces CUDASolver::init (src/solvers/CUDASolver.cpp:52-139). */
+ * to it.  Replaces CUDASolver::init (src/solvers/CUDASolver.cpp:52-139).  Takes
+ * about 420 bytes of device memory a city (320 of them for the neighbour lists)
+ * and the sweep's list of tiles. */
 logo_status logo_ctx_create(int device, const logo_xy *coords, uint32_t n,
                             logo_ctx **out);
 
@@ -306,7 +308,9 @@ typedef struct logo_server logo_server;
 
 typedef struct logo_server_opts {
     int device;
-    uint64_t mem_budget;    /* device bytes for resident requests; 0 = 2 GiB */
+    uint64_t mem_budget;    /* device bytes for resident requests; 0 = 2 GiB (a request above
+                               LOGO_BATCH_MAX_N that does not fit with its neighbour lists
+                               runs without them: 92 bytes a city, graph-driven descents) */
     uint32_t max_slots;     /* requests with n <= LOGO_BATCH_MAX_N in flight; 0 = 4 x SMs */
     uint32_t max_large;     /* larger requests in flight; 0 = 2 */
     uint32_t kicks;         /* ILS kicks per request after its first descent */

@@ -1015,16 +1015,8 @@ float filter_margin(double diag) {
 
 }  // namespace logo
 
-extern "C" {
-
-const char* logo_version(void) { return kVersion; }
-
-const char* logo_last_error(const logo_ctx* ctx) {
-    if (ctx) return ctx->err.c_str();
-    return g_create_err.c_str();
-}
-
-logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_ctx** out) {
+logo_status logo::create_context(int device, const logo_xy* coords, uint32_t n, bool lists,
+                                 logo_ctx** out) {
     if (!out) return fail(nullptr, LOGO_ERR_INVALID_ARG, "out is NULL");
     *out = nullptr;
     if (!coords) return fail(nullptr, LOGO_ERR_INVALID_ARG, "coords is NULL");
@@ -1103,21 +1095,21 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
     CKC(cudaMalloc(&c->d_rbox, sizeof(float4) * sweep_row_windows(n)));
     CKC(cudaMalloc(&c->d_rmax, sizeof(float) * sweep_row_windows(n)));
     CKC(cudaMalloc(&c->d_workctl, 3 * sizeof(uint32_t)));
-    c->solo_ctas = solo_ctas(n, false);
+    c->solo_ctas = lists ? solo_ctas(n, false) : 0;
     c->solo_ils_ctas = c->solo_ctas > 0 ? solo_ctas(n, true) : 0;
     std::memset(c->h_st, 0, sizeof(DevState));
     c->h_st->best_key = kNoMove;
     c->h_st->converged = 1;
     CKC(cudaMemcpyAsync(c->d_st, c->h_st, sizeof(DevState), cudaMemcpyHostToDevice, c->stream));
     CKC(cudaMemcpyAsync(c->d_xy, coords, sizeof(float2) * n, cudaMemcpyHostToDevice, c->stream));
-    c->grid_ctas = near_grid_ctas(n, device);
+    c->grid_ctas = lists ? near_grid_ctas(n, device) : 0;
     if (c->grid_ctas > 0) {
         CKC(cudaMalloc(&c->d_grid, sizeof(GridSync)));
         CKC(cudaMalloc(&c->d_pos, sizeof(uint32_t) * n));
         CKC(cudaMemsetAsync(c->d_pos, 0, sizeof(uint32_t) * n, c->stream));
     }
-    CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n)));
-    near_index_carve(c->near, c->d_near, n);
+    CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n, lists)));
+    near_index_carve(c->near, c->d_near, n, lists);
     search_box(coords, n, x0, y0, x1, y1);
     c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
     s = rebuild(c);
@@ -1126,6 +1118,19 @@ logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_
 #undef CKC
     *out = c;
     return LOGO_OK;
+}
+
+extern "C" {
+
+const char* logo_version(void) { return kVersion; }
+
+const char* logo_last_error(const logo_ctx* ctx) {
+    if (ctx) return ctx->err.c_str();
+    return g_create_err.c_str();
+}
+
+logo_status logo_ctx_create(int device, const logo_xy* coords, uint32_t n, logo_ctx** out) {
+    return create_context(device, coords, n, true, out);
 }
 
 logo_status logo_ctx_destroy(logo_ctx* ctx) {

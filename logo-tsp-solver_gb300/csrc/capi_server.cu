@@ -53,6 +53,7 @@ struct Req {
     std::vector<uint32_t> route;  // start tour, then the result
     ReqState state = kPending;
     bool large = false;
+    bool lists = true;      // a large request: with the descents' neighbour lists
     int slot = -1;
     uint64_t arena_off = 0;
     uint64_t mem = 0;
@@ -104,7 +105,8 @@ constexpr uint64_t kSmallBytesPerCity = sizeof(float2) + 2 * sizeof(uint32_t);
 // device bytes per city of the single-instance path (coordinates, two tour
 // buffers of ordered cities and routes, best tour, the boxed sweep's city
 // positions and near-neighbour lists, and the neighbour lists and cells of the
-// descents); a request that the budget holds but for those last is run alone
+// descents); where the budget has no room for those last, a request runs without
+// them (create_context)
 constexpr uint64_t kLargeLeastBytesPerCity =
     8 + 2 * 16 + 2 * 4 + 16 + 4 + 4 * (1 + kSeedNeighbours);
 constexpr uint64_t kLargeBytesPerCity =
@@ -201,6 +203,7 @@ void run_large(logo_server* s, uint64_t id) {
     std::vector<uint32_t> route;
     uint32_t n;
     uint64_t seed;
+    bool lists;
     {
         std::lock_guard<std::mutex> lk(s->mu);
         Req& r = s->reqs[id];
@@ -208,10 +211,11 @@ void run_large(logo_server* s, uint64_t id) {
         route = r.route;
         n = r.n;
         seed = r.seed;
+        lists = r.lists;
     }
     logo_ctx* ctx = nullptr;
     logo_stats st{};
-    logo_status rc = logo_ctx_create(s->device, xy.data(), n, &ctx);
+    logo_status rc = create_context(s->device, xy.data(), n, lists, &ctx);
     if (rc == LOGO_OK)
         rc = logo_ils(ctx, route.data(), s->opts.kicks, seed, s->opts.kick_kind, &st);
     logo_ctx_destroy(ctx);
@@ -227,7 +231,7 @@ void run_large(logo_server* s, uint64_t id) {
     r.info.status = rc;
     s->mem_in_use -= r.mem;
     s->running_large--;
-    s->running_grid -= r.n > kSoloMaxN;
+    s->running_grid -= r.lists && r.n > kSoloMaxN;
     finish(s, r);
     s->cv.notify_all();
 }
@@ -240,13 +244,13 @@ void admit(logo_server* s) {
         bool ok = false;
         if (r.large) {
             uint64_t mem = kLargeBytesPerCity * r.n;
-            if (mem > s->opts.mem_budget)
-                mem = std::max(kLargeLeastBytesPerCity * r.n, s->opts.mem_budget);
+            r.lists = s->mem_in_use + mem <= s->opts.mem_budget;
+            if (!r.lists) mem = kLargeLeastBytesPerCity * r.n;
             if (s->running_large < s->opts.max_large && s->mem_in_use + mem <= s->opts.mem_budget) {
                 r.mem = mem;
                 s->mem_in_use += mem;
                 s->running_large++;
-                s->running_grid += r.n > kSoloMaxN;
+                s->running_grid += r.lists && r.n > kSoloMaxN;
                 r.state = kRunning;
                 r.t_admit = Clock::now();
                 s->large_ready.push_back(r.id);

@@ -153,9 +153,9 @@ struct NearIndex {
     uint32_t* seeds;  // kSeedNeighbours per city: the lists' first cities (sweep.cu)
     NearGrid g;
 };
-// 32-bit words behind nbr, cell, cellid and seeds.
-size_t near_index_words(uint32_t n);
-void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n);  // words 8-byte aligned
+// 32-bit words behind nbr (null without lists), cell, cellid and seeds.
+size_t near_index_words(uint32_t n, bool lists);
+void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n, bool lists);  // words 8-byte aligned
 // *crowd (pinned host memory): over all cities, the cities of its cell, summed.
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n,
                               unsigned long long* crowd, cudaStream_t s);
@@ -292,6 +292,11 @@ cudaError_t launch_descent_cond(DevState* st, cudaGraphConditionalHandle h, bool
                                 cudaStream_t s);
 cudaError_t launch_kick_cond(DevState* st, cudaGraphConditionalHandle h, bool first,
                              cudaStream_t s);
+
+// logo_ctx_create; without lists the context takes 320 bytes a city less and runs
+// the graph-driven descents, which need none.
+logo_status create_context(int device, const logo_xy* coords, uint32_t n, bool lists,
+                           logo_ctx** out);
 
 // Upper bound of |exact delta - approximate delta| for coordinates whose
 // bounding-box diagonal is `diag` (see filter_margin in capi.cu).

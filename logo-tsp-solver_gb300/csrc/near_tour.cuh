@@ -228,16 +228,15 @@ __device__ __forceinline__ int near_cell(float u, float inv, int cells) {
 }
 
 // ---- the search grid and the neighbour lists ---------------------------------
-// City v's kNearK nearest cities from the filled cells, by one thread: rings of
+// City v's KN nearest cities from the filled cells, by one thread: rings of
 // cells around its own, until the nearest are certain (after ring r every city
 // nearer than r cells has been seen; a little less, for rounding).
 template <typename IX, uint32_t KN>
-__device__ void near_search(uint32_t v, const float2* __restrict__ gxy, const NearGrid& g,
-                            const IX* cell, const IX* cellid, NearEntry<IX>* nbr) {
+__device__ __forceinline__ void near_nearest(uint32_t v, const float2* __restrict__ gxy,
+                                             const NearGrid& g, const IX* cell, const IX* cellid,
+                                             float (&ds)[KN], uint32_t (&vs)[KN]) {
     const float2 p = gxy[v];
     const int cx = near_cell(p.x - g.x0, g.inv, g.gx), cy = near_cell(p.y - g.y0, g.inv, g.gy);
-    float ds[KN];
-    uint32_t vs[KN];
 #pragma unroll
     for (uint32_t k = 0; k < KN; ++k) {
         ds[k] = INFINITY;
@@ -281,6 +280,14 @@ __device__ void near_search(uint32_t v, const float2* __restrict__ gxy, const Ne
             }
         }
     }
+}
+// The same as city v's list.
+template <typename IX, uint32_t KN>
+__device__ void near_search(uint32_t v, const float2* __restrict__ gxy, const NearGrid& g,
+                            const IX* cell, const IX* cellid, NearEntry<IX>* nbr) {
+    float ds[KN];
+    uint32_t vs[KN];
+    near_nearest<IX, KN>(v, gxy, g, cell, cellid, ds, vs);
 #pragma unroll
     for (uint32_t k = 0; k < KN; ++k) {
         NearEntry<IX> e;

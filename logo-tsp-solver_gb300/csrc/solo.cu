@@ -310,6 +310,17 @@ __global__ void near_lists_kernel(const float2* __restrict__ xy, uint32_t n, Nea
         I.seeds[(size_t)v * kSeedNeighbours + k] = I.nbr[(size_t)v * kCtxNear + min(k, n - 2)].x;
 }
 
+// Without lists: the seeds alone.
+__global__ void near_seeds_kernel(const float2* __restrict__ xy, uint32_t n, NearIndex I) {
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    float ds[kSeedNeighbours];
+    uint32_t vs[kSeedNeighbours];
+    near_nearest<uint32_t, kSeedNeighbours>(v, xy, I.g, I.cell, I.cellid, ds, vs);
+    for (uint32_t k = 0; k < kSeedNeighbours; ++k)
+        I.seeds[(size_t)v * kSeedNeighbours + k] = vs[min(k, n - 2)];
+}
+
 void solo_config(uint32_t n, int nt, uint32_t ctas, cudaLaunchConfig_t* cfg,
                  cudaLaunchAttribute* attr, cudaStream_t s) {
     *cfg = cudaLaunchConfig_t{};
@@ -379,30 +390,39 @@ cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s) {
     return ils ? launch_solo_t<512, true>(A, ctas, s) : launch_solo_t<512, false>(A, ctas, s);
 }
 
-size_t near_index_words(uint32_t n) {
-    // lists (also the sort's counters), cells and their end, cities by cell, seeds
-    return std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n)) + near_cells_max(n) + 1 +
-           (size_t)n * (1 + kSeedNeighbours);
+// Words of the lists, or without them of the seeds; either holds the sort's counters first.
+static size_t near_first_words(uint32_t n, bool lists) {
+    return std::max<size_t>((size_t)n * (lists ? kCtxNear * 2 : kSeedNeighbours),
+                            near_cells_max(n));
 }
 
-void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n) {
-    I.nbr = reinterpret_cast<uint2*>(words);
-    I.cell = words + std::max<size_t>((size_t)n * kCtxNear * 2, near_cells_max(n));
+size_t near_index_words(uint32_t n, bool lists) {
+    // lists, cells and their end, cities by cell, seeds
+    return near_first_words(n, lists) + near_cells_max(n) + 1 + n +
+           (lists ? (size_t)n * kSeedNeighbours : 0);
+}
+
+void near_index_carve(NearIndex& I, uint32_t* words, uint32_t n, bool lists) {
+    I.nbr = lists ? reinterpret_cast<uint2*>(words) : nullptr;
+    I.cell = words + near_first_words(n, lists);
     I.cellid = I.cell + near_cells_max(n) + 1;
-    I.seeds = I.cellid + n;
+    I.seeds = lists ? I.cellid + n : words;
 }
 
 cudaError_t launch_near_index(const NearIndex& I, const float2* xy, uint32_t n,
                               unsigned long long* crowd, cudaStream_t s) {
     const uint32_t cells = (uint32_t)I.g.gx * (uint32_t)I.g.gy;
     const uint32_t grid = (n + 255) / 256;
-    uint32_t* count = reinterpret_cast<uint32_t*>(I.nbr);
+    uint32_t* count = I.nbr ? reinterpret_cast<uint32_t*>(I.nbr) : I.seeds;
     cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t) * cells, s);
     if (e != cudaSuccess) return e;
     near_count_kernel<<<grid, 256, 0, s>>>(xy, n, I.g, count);
     near_scan_kernel<<<1, 1024, 0, s>>>(count, I.cell, cells, crowd);
     near_scatter_kernel<<<grid, 256, 0, s>>>(xy, n, I.g, count, I.cellid);
-    near_lists_kernel<<<(n + 127) / 128, 128, 0, s>>>(xy, n, I);
+    if (I.nbr)
+        near_lists_kernel<<<(n + 127) / 128, 128, 0, s>>>(xy, n, I);
+    else
+        near_seeds_kernel<<<(n + 127) / 128, 128, 0, s>>>(xy, n, I);
     return cudaGetLastError();
 }
 

@@ -20,3 +20,35 @@ def test_grid_wide_requests_and_rounds(lg, inst):
         for route, info in (got[k], got[k + len(reqs)]):
             assert info["status"] == 0 and info["best_length"] == st["final_length"]
             assert info["moves"] == st["moves"] and np.array_equal(route, want)
+
+
+def test_large_requests_within_a_small_budget(lg, inst):
+    """A budget without room for a large request's neighbour lists holds the
+    request without them: it is charged what it takes and need not wait for the
+    others to end."""
+    n = 7000
+    xy = inst.uniform_f32(n, 81, 1.0e5)
+    r = lg.nn_tour(xy)
+    small = inst.uniform_f32(4000, 82, 1.0e5)
+    rs = inst.random_tour(4000, 83)
+    with lg.Solver(xy) as s:
+        want, st = s.ils(r, 3, 5, lg.KICK_SEGMENT)
+    budget = 92 * n + 3 * 16 * 4000
+    with lg.Server(kicks=3, mem_budget=budget, quantum_pairs=100_000) as srv:
+        busy = [srv.submit(small, rs, k) for k in range(2)]
+        rid = srv.submit(xy, r, 5)
+        seen = set()
+        while True:
+            info = srv.stats()
+            assert info["mem_in_use"] <= budget
+            if info["running_large"]:
+                seen.add((info["mem_in_use"], info["running_small"]))
+            got = srv.poll(rid)
+            if got is not None:
+                break
+        for k in busy:
+            srv.wait(k)
+    assert got[1]["status"] == 0 and got[1]["best_length"] == st["final_length"]
+    assert got[1]["moves"] == st["moves"] and np.array_equal(got[0], want)
+    # beside the small requests that came first
+    assert (92 * n + 2 * 16 * 4000, 2) in seen, seen
