@@ -600,12 +600,15 @@ logo_status logo_diag_wait_limits(int device, uint32_t *mbarrier_status,
 logo_status logo_diag_flag_timeout(logo_ctx *ctx);
 
 /* Test hooks of the grid-wide launch (tours above 6,144 cities): how many edges
- * put off in a sweep it lists, how many edges it lists for their pairs, and from
- * how many cities a disc is put off (0: the library's own limits, which are also
- * the largest); results never depend on them.  The counts are the largest of any
- * sweep of the context's last such launch. */
-logo_status logo_diag_grid_limits(logo_ctx *ctx, uint32_t wide, uint32_t takers, uint32_t disc);
-logo_status logo_diag_grid_counts(logo_ctx *ctx, uint32_t *wide, uint32_t *takers);
+ * put off in a sweep it lists, how many edges it lists for their pairs, above how
+ * many cities a disc is put off as edges, and how many discs it lists that are dealt
+ * to the whole device (0: the library's own limits, which are also the largest, and
+ * discs dealt above 50,000 cities only); results never depend on them.  The counts
+ * are the largest of any sweep of the context's last such launch. */
+logo_status logo_diag_grid_limits(logo_ctx *ctx, uint32_t wide, uint32_t takers, uint32_t disc,
+                                  uint32_t discs);
+logo_status logo_diag_grid_counts(logo_ctx *ctx, uint32_t *wide, uint32_t *takers,
+                                  uint32_t *discs);
 /* Test hook: after how many microseconds a grid-wide launch ends between two moves
  * to let other work onto the device (0: the default, 20000); results never depend on
  * it. */

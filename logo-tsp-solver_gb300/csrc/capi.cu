@@ -64,6 +64,7 @@ struct logo_ctx {
     int grid_ctas = 0;            // CTAs of the grid-wide descent of larger tours (0: unavailable)
     GridSync* d_grid = nullptr;
     uint32_t grid_wide = kGridWide, grid_takers = kGridTakers, grid_disc = kGridDisc;
+    uint32_t grid_discs = kGridDiscs, grid_spread = kGridSpread;
     unsigned long long grid_quantum_ns = kGridQuantumNs;
     bool own_kernel = false;      // the caller chose a sweep kernel: descents run that one
     int descent_mode = LOGO_DESCENT_AUTO;
@@ -199,6 +200,8 @@ GridArgs grid_args(const logo_ctx* c) {
     A.wide = c->grid_wide;
     A.takers = c->grid_takers;
     A.disc = c->grid_disc;
+    A.discs = c->grid_discs;
+    A.spread = c->grid_spread;
     A.quantum_ns = c->grid_quantum_ns;
     return A;
 }
@@ -1323,26 +1326,31 @@ logo_status logo_diag_flag_timeout(logo_ctx* c) {
     return LOGO_OK;
 }
 
-logo_status logo_diag_grid_limits(logo_ctx* c, uint32_t wide, uint32_t takers, uint32_t disc) {
+logo_status logo_diag_grid_limits(logo_ctx* c, uint32_t wide, uint32_t takers, uint32_t disc,
+                                  uint32_t discs) {
     if (!c) return LOGO_ERR_INVALID_ARG;
-    if (wide > kGridWide || takers > kGridTakers || disc > kGridDisc)
+    if (wide > kGridWide || takers > kGridTakers || disc > kGridDisc || discs > kGridDiscs)
         return fail(c, LOGO_ERR_INVALID_ARG, "above the library's own limits");
     c->grid_wide = wide ? wide : kGridWide;
     c->grid_takers = takers ? takers : kGridTakers;
     c->grid_disc = disc ? disc : kGridDisc;
+    c->grid_discs = discs ? discs : kGridDiscs;
+    c->grid_spread = discs ? 0u : kGridSpread;
     return LOGO_OK;
 }
 
-logo_status logo_diag_grid_counts(logo_ctx* c, uint32_t* wide, uint32_t* takers) {
-    if (!c || !wide || !takers) return LOGO_ERR_INVALID_ARG;
+logo_status logo_diag_grid_counts(logo_ctx* c, uint32_t* wide, uint32_t* takers,
+                                  uint32_t* discs) {
+    if (!c || !wide || !takers || !discs) return LOGO_ERR_INVALID_ARG;
     if (!c->d_grid) return fail(c, LOGO_ERR_INVALID_ARG, "no grid-wide launches at this size");
     CK(c, cudaSetDevice(c->device));
-    uint32_t most[2] = {0u, 0u};
+    uint32_t most[3] = {0u, 0u, 0u};
     CK(c, cudaMemcpyAsync(most, &c->d_grid->most_wides, sizeof(most), cudaMemcpyDeviceToHost,
                           c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     *wide = most[0];
     *takers = most[1];
+    *discs = most[2];
     return LOGO_OK;
 }
 

@@ -19,6 +19,14 @@
 // of a 100,000-city route: 111 -> 60 us; best move of 1,000,000: 612 -> 168 us,
 // most of it the route's way from host memory).
 //
+// Up to A.spread cities a CTA goes through its large discs itself, above (SPREAD) they
+// are dealt to all CTAs after one more barrier: with more slots a CTA, one had up to
+// 20 discs while the others waited (best move of an NN tour of n = 100,000: 95 -> 66
+// us, of 1,000,000: 247 -> 165; of a random one 81 -> 66 and 163 -> 109; a sweep early
+// in a descent of n = 100,000: 57 -> 43.  Below, the barrier costs more: n = 20,000
+// clustered 23 -> 26 us a sweep, 1 of it by the kernel's size alone, so there are two;
+// n = 40,009 35 -> 35, later in the descent 26 -> 31).
+//
 // Discs of more than kGridDisc cities (long edges of a tour far from a local
 // optimum) are put off to all CTAs: the few edges against every edge that can
 // take part, after one more barrier.  One CTA going through them held up the rest
@@ -106,14 +114,14 @@ __device__ __forceinline__ bool grid_load(GridTour& T, const SoloArgs& A,
     return bad;
 }
 
-template <bool ILS>
+template <bool ILS, bool SPREAD>
 __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     constexpr int NT = kGridNT, NW = NT / 32;
     __shared__ NearShared<NT, 1, uint32_t> S;
     __shared__ bool bar_ok;
     __shared__ uint2 seeds[32];
     __shared__ unsigned long long best_key;
-    __shared__ uint32_t wide_count, pause_now;
+    __shared__ uint32_t wide_count, disc_count, pause_now;
     DevState* st = A.solo.st;
     const bool whole = !ILS && A.solo.call.src != nullptr;
     // set before the launch and identical for every CTA
@@ -192,7 +200,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     unsigned long long m = 0, sweeps = 0, total_m = 0;
     unsigned long long best_len = 0, accepted = 0, kicks = 0;
     uint64_t rng = 0;
-    uint32_t most_wides = 0, most_takers = 0;
+    uint32_t most_wides = 0, most_takers = 0, most_discs = 0;
     if (ILS) {
         best_len = *(volatile unsigned long long*)&st->best_length;
         rng = *(volatile unsigned long long*)&st->rng;
@@ -201,75 +209,108 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     for (uint32_t it = ILS ? (uint32_t)*(volatile unsigned long long*)&st->kicks : 0u; ok; ++it) {
         m = 0;
         for (;;) {
-            NearBest nb{near_scan<NT, false>(T, S, seed, parity, rank, ranks, A.disc), -1.f};
+            NearBest nb{near_scan<NT, false, SPREAD>(T, S, seed, parity, rank, ranks, A.disc),
+                        -1.f};
             const uint32_t z = T.closing();
             __syncthreads();
-            const uint32_t huges = S.huges[parity];  // the same for every thread
+            // (the same for every thread)
+            const uint32_t huges = SPREAD ? min(S.big[parity], kNearWide) : S.huges[parity];
             if (huges) {
-                // the edges of these slots that reach beyond their lists
                 // (the CTA's bound, not the lane's own best: near_far wants one for the warp)
                 nb.B = fminf((float)S.bound[parity], (float)S.far_bound[parity]);
                 const float h = near_half((float)S.bound[parity]);
-                for (uint32_t o = warp; o < 2 * huges; o += NW) {
-                    const uint32_t j = S.huge[o / 2], f = o & 1 ? T.wrap(j + 1) : j;
-                    if (f == z || T.last_sq(j) > near_limit(T.E[f] + h)) continue;
-                    uint32_t at = 0;
-                    if (lane == 0) at = atomicAdd(&A.gs->wides[parity], 1u);
-                    at = __shfl_sync(0xffffffffu, at, 0);
-                    if (at >= A.wide)
-                        near_far(T, j, z, ~0u, nb.B, nb);  // no room for this one
-                    else if (lane == 0)
-                        A.gs->wide[parity][at] = f;
+                for (uint32_t o = warp; o < huges; o += NW) {
+                    const uint32_t j = SPREAD ? S.wide[o] : S.huge[o];
+                    // its disc, or where that is too large its edges that reach beyond its list
+                    const bool disc = SPREAD && !near_large(T, j, z, A.disc, nb.B);
+#pragma unroll 1
+                    for (uint32_t s = 0; s < (disc ? 1u : 2u); ++s) {
+                        const uint32_t f = s ? T.wrap(j + 1) : j;
+                        if (!disc && (f == z || T.last_sq(j) > near_limit(T.E[f] + h))) continue;
+                        uint32_t at = 0;
+                        if (lane == 0)
+                            at = atomicAdd(disc ? &A.gs->discs[parity] : &A.gs->wides[parity], 1u);
+                        at = __shfl_sync(0xffffffffu, at, 0);
+                        if (at >= (disc ? A.discs : A.wide))
+                            near_far(T, j, z, ~0u, nb.B, nb);  // no room for this one
+                        else if (lane == 0)
+                            (disc ? A.gs->disc[parity] : A.gs->wide[parity])[at] = f;
+                    }
                 }
             }
-            if (tid == 0) A.gs->pause[parity] = global_timer_ns() - begun > A.quantum_ns;
+            // (the clock is slow to read)
+            if (tid == 0 && ((sweeps & 15u) == 15u || A.quantum_ns < 1000000u) &&
+                global_timer_ns() - begun > A.quantum_ns)
+                A.gs->pause[parity] = 1u;
             publish(A.gs->keys[parity], nb.key);
             if (!(ok = barrier())) break;
             ++sweeps;
-            if (tid == 0) A.gs->wides[parity ^ 1] = A.gs->takers[parity ^ 1] = 0;  // the next sweep's
+            if (tid == 0) {  // the next sweep's
+                A.gs->wides[parity ^ 1] = A.gs->takers[parity ^ 1] = 0;
+                if (SPREAD) A.gs->discs[parity ^ 1] = 0;
+            }
             // one warp per CTA reads the keys (all of them reading the same few
             // lines queued up at L2 for 7 us)
             if (warp == 0) {
                 const uint32_t w = *(volatile uint32_t*)&A.gs->wides[parity];
+                const uint32_t d = SPREAD ? *(volatile uint32_t*)&A.gs->discs[parity] : 0u;
                 const uint32_t pause = *(volatile uint32_t*)&A.gs->pause[parity];
                 const uint64_t k = near_pick(T, A.gs->keys[parity], ranks, seed);
                 seeds[lane] = make_uint2(seed.a, seed.b);
                 if (lane == 0) {
                     best_key = k;
                     wide_count = w;
+                    if (SPREAD) disc_count = d;
                     pause_now = pause;
                 }
             }
             __syncthreads();
             uint64_t key = best_key;
             const uint32_t wides = min(wide_count, A.wide);
+            const uint32_t discs = SPREAD ? min(disc_count, A.discs) : 0u;
             most_wides = max(most_wides, wide_count);
-            if (wides) {
+            if (wides || discs) {
+                const float known = key == kNoMove ? -1.f : (float)key_delta(key);
+                NearBest more{key, known};
+                if constexpr (SPREAD) {
+                    // discs put off, a CTA each
+                    most_discs = max(most_discs, disc_count);
+                    for (uint32_t d = rank; d < discs; d += ranks) {
+                        const uint32_t j = A.gs->disc[parity][d], jn = T.wrap(j + 1);
+                        const float m =
+                            fmaxf(j == z ? kNoEdge : T.E[j], jn == z ? kNoEdge : T.E[jn]);
+                        if (2.f * m + 8.f >= -known &&
+                            T.last_sq(j) <= near_limit(m + near_half(known)))
+                            near_far(T, j, z, ~0u, known, more, warp, NW);
+                    }
+                }
                 // edges put off, with every edge that can take part: listed first,
                 // so that the pairs can be dealt evenly, unless those are too many
-                NearBest more{key, key == kNoMove ? -1.f : (float)key_delta(key)};
-                for (uint32_t base = tid - lane; base < n; base += threads) {
-                    const uint32_t g = base + lane;
-                    const bool takes = g < n && g != z && 2.f * T.E[g] + 8.f >= -more.B;
-                    const uint32_t votes = __ballot_sync(0xffffffffu, takes);
-                    if (votes == 0) continue;
-                    uint32_t at = 0;
-                    if (lane == 0) at = atomicAdd(&A.gs->takers[parity], (uint32_t)__popc(votes));
-                    at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1u));
-                    if (takes && at < A.takers) A.gs->taker[at] = g;
-                }
-                if (!(ok = barrier())) break;
-                const uint32_t takers = *(volatile uint32_t*)&A.gs->takers[parity];
-                most_takers = max(most_takers, takers);
-                if (takers <= A.takers) {
-                    for (uint32_t base = tid - lane; base < wides * takers; base += threads) {
-                        const uint32_t t = base + lane;
-                        const bool in = t < wides * takers;
-                        near_edges(T, &A.gs->wide[parity][in ? t / takers : 0], 1u, in,
-                                   A.gs->taker[in ? t % takers : 0], z, more);
+                if (wides) {
+                    for (uint32_t base = tid - lane; base < n; base += threads) {
+                        const uint32_t g = base + lane;
+                        const bool takes = g < n && g != z && 2.f * T.E[g] + 8.f >= -known;
+                        const uint32_t votes = __ballot_sync(0xffffffffu, takes);
+                        if (votes == 0) continue;
+                        uint32_t at = 0;
+                        if (lane == 0)
+                            at = atomicAdd(&A.gs->takers[parity], (uint32_t)__popc(votes));
+                        at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1u));
+                        if (takes && at < A.takers) A.gs->taker[at] = g;
                     }
-                } else {
-                    grid_edges(T, A.gs->wide[parity], wides, z, more, tid, threads);
+                    if (!(ok = barrier())) break;
+                    const uint32_t takers = *(volatile uint32_t*)&A.gs->takers[parity];
+                    most_takers = max(most_takers, takers);
+                    if (takers <= A.takers) {
+                        for (uint32_t base = tid - lane; base < wides * takers; base += threads) {
+                            const uint32_t t = base + lane;
+                            const bool in = t < wides * takers;
+                            near_edges(T, &A.gs->wide[parity][in ? t / takers : 0], 1u, in,
+                                       A.gs->taker[in ? t % takers : 0], z, more);
+                        }
+                    } else {
+                        grid_edges(T, A.gs->wide[parity], wides, z, more, tid, threads);
+                    }
                 }
                 publish(A.gs->wide_keys[parity], more.key);
                 if (!(ok = barrier())) break;
@@ -398,14 +439,15 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
         st->converged = (step || paused) && ok ? 0u : 1u;
         A.gs->most_wides = most_wides;
         A.gs->most_takers = most_takers;
+        A.gs->most_discs = most_discs;
     }
     if (whole) leave();
 }
 
-template <bool ILS>
+template <bool ILS, bool SPREAD>
 int grid_ctas_t(int device) {
     int per_sm = 0, sms = 0, coop = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, near_grid_kernel<ILS>, kGridNT, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, near_grid_kernel<ILS, SPREAD>, kGridNT, 0) !=
             cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess)
@@ -417,7 +459,8 @@ int grid_ctas_t(int device) {
 
 int near_grid_ctas(uint32_t n, int device) {
     if (n <= kSoloMaxN) return 0;
-    return std::min(grid_ctas_t<false>(device), grid_ctas_t<true>(device));
+    return std::min({grid_ctas_t<false, false>(device), grid_ctas_t<true, false>(device),
+                     grid_ctas_t<false, true>(device), grid_ctas_t<true, true>(device)});
 }
 
 cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t s) {
@@ -432,8 +475,11 @@ cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (ils) return cudaLaunchKernelEx(&cfg, near_grid_kernel<true>, A);
-    return cudaLaunchKernelEx(&cfg, near_grid_kernel<false>, A);
+    if (A.solo.n > A.spread)
+        return ils ? cudaLaunchKernelEx(&cfg, near_grid_kernel<true, true>, A)
+                   : cudaLaunchKernelEx(&cfg, near_grid_kernel<false, true>, A);
+    return ils ? cudaLaunchKernelEx(&cfg, near_grid_kernel<true, false>, A)
+               : cudaLaunchKernelEx(&cfg, near_grid_kernel<false, false>, A);
 }
 
 }  // namespace logo

@@ -207,6 +207,8 @@ cudaError_t launch_solo(const SoloArgs& A, bool ils, int ctas, cudaStream_t s);
 constexpr uint32_t kGridMaxCtas = 256;
 constexpr uint32_t kGridWide = 1024, kGridTakers = 8192;
 constexpr uint32_t kGridDisc = 4096;  // cities of a disc that one CTA goes through
+constexpr uint32_t kGridDiscs = 4096;  // discs put off that are listed
+constexpr uint32_t kGridSpread = 50000;  // default of GridArgs::spread (see grid_tour.cu)
 struct GridSync {
     unsigned long long arrived;    // barrier arrivals so far
     unsigned long long length[2];  // tour length of the descent in hand, by its parity
@@ -215,20 +217,23 @@ struct GridSync {
     // edges put off in a sweep, and edges that can take part in pairs with them,
     // by its parity (more may have been offered than fit)
     uint32_t wides[2], takers[2];
+    uint32_t discs[2];  // slots whose discs are put off, likewise
     uint32_t left;  // CTAs that have left a whole call
     uint32_t pause[2];  // the launch is to end after this sweep's move, by its parity
     // (set to zero up to here before a launch)
     unsigned long long wide_keys[2][kGridMaxCtas];  // best key per CTA after those
     uint32_t wide[2][kGridWide];
+    uint32_t disc[2][kGridDiscs];
     uint32_t taker[kGridTakers];
     unsigned long long keys[2][kGridMaxCtas];  // best key per CTA, by the sweep's parity
-    uint32_t most_wides, most_takers;  // largest counts of a sweep of the last launch
+    uint32_t most_wides, most_takers, most_discs;  // largest counts of a sweep of the last launch
 };
 struct GridArgs {
     SoloArgs solo;  // pos: slot of every city meanwhile
     GridSync* gs;
-    // limits, at most (a test's are smaller) kGridWide, kGridTakers and kGridDisc
-    uint32_t wide, takers, disc;
+    // limits, at most (a test's are smaller) kGridWide, kGridTakers, kGridDisc, kGridDiscs
+    uint32_t wide, takers, disc, discs;
+    uint32_t spread;  // tours above as many cities have their large discs dealt to all CTAs
     unsigned long long quantum_ns;  // a launch that has run for longer ends after its next move
 };
 // Default of quantum_ns: how long other work on the device (another context's call, a

@@ -586,6 +586,25 @@ __device__ __forceinline__ bool near_meet(const TOUR& T, bool in, uint32_t j, ui
     return met;
 }
 
+// Whether the disc of slot j under bound B has more than `most` cities (as near_far
+// sees it); the whole warp, j and B the same in every lane.
+template <typename TOUR>
+__device__ __forceinline__ bool near_large(const TOUR& T, uint32_t j, uint32_t z, uint32_t most,
+                                           float B) {
+    const uint32_t jn = T.wrap(j + 1);
+    const float ej = j == z ? kNoEdge : T.E[j], en = jn == z ? kNoEdge : T.E[jn];
+    const float V = fmaxf(ej, en) + near_half(B), r = V + 2.f;
+    if (V < 0.f) return false;
+    const float ux = T.xy[j].x - T.g.x0, uy = T.xy[j].y - T.g.y0;
+    const int xa = near_cell(ux - r, T.g.inv, T.g.gx), xb = near_cell(ux + r, T.g.inv, T.g.gx);
+    const int ya = near_cell(uy - r, T.g.inv, T.g.gy), yb = near_cell(uy + r, T.g.inv, T.g.gy);
+    if (2u * (uint32_t)((xb - xa + 1) * (yb - ya + 1)) > most) return true;
+    uint32_t held = 0;
+    for (int y = ya + (int)(threadIdx.x & 31); y <= yb; y += 32)
+        held += T.cell[y * T.g.gx + xb + 1] - T.cell[y * T.g.gx + xa];
+    return __reduce_add_sync(0xffffffffu, held) > most;
+}
+
 // A slot whose list was too short, looked at by the whole warp: the grid's
 // cells in the disc that bound B gives, of whose cities this warp takes part
 // `part` of `parts` (B has to be the same in all of those warps: they number the
@@ -804,8 +823,9 @@ __device__ __forceinline__ uint32_t near_lists(const TOUR& T, SLOTS& w, uint32_t
 // 4. Large discs are put off to all warps of the CTA, which take a part each
 //    (those beyond `huge` stay in S.huge for the caller), or with ALL_EDGES go
 //    over the edges that can take part instead (long edges of a tour far from a
-//    local optimum: the bound is large then, and most edges too short).
-template <int NT, bool ALL_EDGES, typename TOUR, typename SH>
+//    local optimum: the bound is large then, and most edges too short).  With LEAVE
+//    they stay in S.wide for the caller.
+template <int NT, bool ALL_EDGES, bool LEAVE = false, typename TOUR, typename SH>
 __device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSeed& seed,
                                               uint32_t parity, uint32_t rank, uint32_t ranks,
                                               uint32_t huge = ~0u) {
@@ -911,6 +931,7 @@ __device__ __forceinline__ uint64_t near_scan(const TOUR& T, SH& S, const NearSe
         if (lane == 0 && nb.B < list_bound) atomicMin(&S.far_bound[parity], (int)nb.B);
     }
     __syncthreads();
+    if (LEAVE) return nb.key;
     const uint32_t big = min(S.big[parity], kNearWide);  // the same for every thread
     const float bound = fminf(list_bound, (float)S.far_bound[parity]);
     nb.B = fminf(nb.B, bound);

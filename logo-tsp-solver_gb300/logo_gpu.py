@@ -193,8 +193,8 @@ def load(path=LIB_PATH):
                                      c.c_uint64, c.POINTER(Stats)]
     L.logo_diag_sqrt_error.argtypes = [c.c_int, ctypes.POINTER(ctypes.c_double)]
     L.logo_diag_flag_timeout.argtypes = [_vp]
-    L.logo_diag_grid_limits.argtypes = [_vp, c.c_uint32, c.c_uint32, c.c_uint32]
-    L.logo_diag_grid_counts.argtypes = [_vp, _u32p, _u32p]
+    L.logo_diag_grid_limits.argtypes = [_vp, c.c_uint32, c.c_uint32, c.c_uint32, c.c_uint32]
+    L.logo_diag_grid_counts.argtypes = [_vp, _u32p, _u32p, _u32p]
     L.logo_diag_grid_quantum.argtypes = [_vp, c.c_uint32]
     L.logo_diag_wait_limits.argtypes = [c.c_int, ctypes.POINTER(ctypes.c_uint32),
                                         ctypes.POINTER(ctypes.c_uint32),
@@ -431,20 +431,21 @@ class Solver:
         would (logo_diag_flag_timeout)."""
         _check(load().logo_diag_flag_timeout(self._h), self._h)
 
-    def grid_limits(self, wide=0, takers=0, disc=0):
+    def grid_limits(self, wide=0, takers=0, disc=0, discs=0):
         """Test hook: limits of the grid-wide launch (logo_diag_grid_limits)."""
-        _check(load().logo_diag_grid_limits(self._h, wide, takers, disc), self._h)
+        _check(load().logo_diag_grid_limits(self._h, wide, takers, disc, discs), self._h)
 
     def grid_quantum(self, us=0):
         """Test hook: when a grid-wide launch pauses (logo_diag_grid_quantum)."""
         _check(load().logo_diag_grid_quantum(self._h, us), self._h)
 
     def grid_counts(self):
-        """Test hook: most edges put off and most edges listed for them in a
-        sweep of the last grid-wide launch (logo_diag_grid_counts)."""
-        a, b = ctypes.c_uint32(), ctypes.c_uint32()
-        _check(load().logo_diag_grid_counts(self._h, ctypes.byref(a), ctypes.byref(b)), self._h)
-        return a.value, b.value
+        """Test hook: most edges put off, most edges listed for them and most
+        discs put off in a sweep of the last grid-wide launch
+        (logo_diag_grid_counts)."""
+        v = [ctypes.c_uint32() for _ in range(3)]
+        _check(load().logo_diag_grid_counts(self._h, *[ctypes.byref(x) for x in v]), self._h)
+        return tuple(x.value for x in v)
 
 
 def read_tsplib(path):

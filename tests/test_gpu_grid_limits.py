@@ -8,8 +8,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# (edges put off, edges listed for their pairs, cities of a disc)
-@pytest.mark.parametrize("limits", [(0, 0, 64), (2, 0, 64), (0, 8, 64), (2, 8, 64), (1, 1, 1)])
+# (edges put off, edges listed for their pairs, cities of a disc, discs put off)
+@pytest.mark.parametrize("limits", [(0, 0, 64, 0), (2, 0, 64, 0), (0, 8, 64, 0), (2, 8, 64, 0),
+                                    (1, 1, 1, 0), (0, 0, 64, 4096), (2, 8, 64, 1)])
 @pytest.mark.parametrize("points", ["uniform", "clustered"])
 def test_more_edges_than_the_lists_hold(lg, inst, points, limits):
     n = 7000
@@ -23,7 +24,7 @@ def test_more_edges_than_the_lists_hold(lg, inst, points, limits):
     with lg.Solver(xy) as s:
         s.grid_limits(*limits)
         got, trace, gst = s.optimize_trace(r, max_moves=250)
-        wides, takers = s.grid_counts()
+        wides, takers, _ = s.grid_counts()
         # the branches under test were taken: edges were put off, more than are listed
         assert wides > limits[0] and takers > limits[1]
         assert np.array_equal(trace, log) and np.array_equal(got, want)
@@ -35,12 +36,12 @@ def test_more_edges_than_the_lists_hold(lg, inst, points, limits):
 
 def test_limits_above_the_lists_are_refused(lg, inst):
     with lg.Solver(inst.uniform_f32(7000, 1, 1.0e4)) as s:
-        for limits in ((1025, 0, 0), (0, 8193, 0), (0, 0, 4097)):
+        for limits in ((1025, 0, 0, 0), (0, 8193, 0, 0), (0, 0, 4097, 0), (0, 0, 0, 4097)):
             with pytest.raises(lg.LogoError):
                 s.grid_limits(*limits)
 
 
-def both_ways(lg, xy, r, moves, limits=(0, 0, 0)):
+def both_ways(lg, xy, r, moves, limits=(0, 0, 0, 0)):
     res = []
     for mode in (lg.DESCENT_GRAPH, lg.DESCENT_AUTO):
         with lg.Solver(xy) as s:
@@ -59,7 +60,26 @@ def test_a_disc_is_counted_by_its_cities(lg, inst):
     of one cell holds thousands of cities and has to be put off."""
     xy = inst.uniform_f32(7000, 11, 100.0)
     xy[::2] += np.float32(1.0e6)
-    assert both_ways(lg, xy, lg.nn_tour(xy), 120, limits=(0, 0, 1024))[0] > 0
+    assert both_ways(lg, xy, lg.nn_tour(xy), 120, limits=(0, 0, 1024, 0))[0] > 0
+
+
+@pytest.mark.parametrize("discs", [4096, 3])
+@pytest.mark.parametrize("n,kind", [(6145, "uniform"), (7000, "clustered"), (20000, "uniform"),
+                                    (20000, "clustered")])
+def test_discs_dealt_to_all_ctas(lg, inst, n, kind, discs):
+    """As above 50,000 cities; from a nearest-neighbour and a random tour, and
+    with more of them than are listed."""
+    xy = (inst.clustered(n, n, clusters=20, sigma_frac=0.03) if kind == "clustered"
+          else inst.uniform_f32(n, n, 1.0e5))
+    assert both_ways(lg, xy, lg.nn_tour(xy), 300, limits=(0, 0, 0, discs))[2] > discs % 4096
+    both_ways(lg, xy, inst.random_tour(n, 1), 80, limits=(0, 0, 0, discs))
+
+
+@pytest.mark.parametrize("n", [50001, 100003])
+def test_above_the_size_where_discs_are_dealt(lg, inst, n):
+    xy = inst.clustered(n, 3)
+    assert both_ways(lg, xy, lg.nn_tour(xy), 60)[2] > 0
+    both_ways(lg, xy, inst.random_tour(n, 1), 20)
 
 
 @pytest.mark.parametrize("kind", ["stray", "strays", "heaps"])
