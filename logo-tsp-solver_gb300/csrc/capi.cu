@@ -63,6 +63,7 @@ struct logo_ctx {
     int solo_ils_ctas = 0;        // the same for a whole ILS call
     int grid_ctas = 0;            // CTAs of the grid-wide descent of larger tours (0: unavailable)
     GridSync* d_grid = nullptr;
+    uint32_t* d_grid_disc = nullptr;  // (behind d_near's arrays)
     uint32_t grid_wide = kGridWide, grid_takers = kGridTakers, grid_disc = kGridDisc;
     uint32_t grid_discs = kGridDiscs, grid_spread = kGridSpread;
     unsigned long long grid_quantum_ns = kGridQuantumNs;
@@ -197,6 +198,7 @@ GridArgs grid_args(const logo_ctx* c) {
     GridArgs A{};
     A.solo = solo_args(c);
     A.gs = c->d_grid;
+    A.disc_list = c->d_grid_disc;
     A.wide = c->grid_wide;
     A.takers = c->grid_takers;
     A.disc = c->grid_disc;
@@ -1111,7 +1113,10 @@ logo_status logo::create_context(int device, const logo_xy* coords, uint32_t n, 
         CKC(cudaMalloc(&c->d_pos, sizeof(uint32_t) * n));
         CKC(cudaMemsetAsync(c->d_pos, 0, sizeof(uint32_t) * n, c->stream));
     }
-    CKC(cudaMalloc(&c->d_near, sizeof(uint32_t) * near_index_words(n, lists)));
+    const size_t near_words = near_index_words(n, lists);
+    CKC(cudaMalloc(&c->d_near,
+                   sizeof(uint32_t) * (near_words + (c->grid_ctas > 0 ? 2 * kGridDiscs : 0))));
+    c->d_grid_disc = c->d_near + near_words;
     near_index_carve(c->near, c->d_near, n, lists);
     search_box(coords, n, x0, y0, x1, y1);
     c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));

@@ -122,6 +122,9 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     __shared__ uint2 seeds[32];
     __shared__ unsigned long long best_key;
     __shared__ uint32_t wide_count, disc_count, pause_now;
+    // (in shared memory for the sweep's registers; one thread uses them)
+    __shared__ uint32_t most[3];
+    __shared__ unsigned long long begun;
     DevState* st = A.solo.st;
     const bool whole = !ILS && A.solo.call.src != nullptr;
     // set before the launch and identical for every CTA
@@ -129,7 +132,10 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     const uint32_t n = A.solo.n, rank = blockIdx.x, ranks = gridDim.x;
     const uint32_t tid = rank * NT + threadIdx.x, threads = ranks * NT;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned long long begun = tid == 0 ? global_timer_ns() : 0ull;
+    if (threadIdx.x == 0) {
+        begun = global_timer_ns();
+        most[0] = most[1] = most[2] = 0;
+    }
     const uint32_t cur = whole ? 0u : *(volatile unsigned int*)&st->cur;
     OrderedCity* Qg = cur ? A.solo.Q1 : A.solo.Q0;
     uint32_t* Rg = cur ? A.solo.R1 : A.solo.R0;
@@ -200,7 +206,6 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
     unsigned long long m = 0, sweeps = 0, total_m = 0;
     unsigned long long best_len = 0, accepted = 0, kicks = 0;
     uint64_t rng = 0;
-    uint32_t most_wides = 0, most_takers = 0, most_discs = 0;
     if (ILS) {
         best_len = *(volatile unsigned long long*)&st->best_length;
         rng = *(volatile unsigned long long*)&st->rng;
@@ -212,6 +217,7 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             NearBest nb{near_scan<NT, false, SPREAD>(T, S, seed, parity, rank, ranks, A.disc),
                         -1.f};
             const uint32_t z = T.closing();
+            auto& put = A.gs->put[parity];
             __syncthreads();
             // (the same for every thread)
             const uint32_t huges = SPREAD ? min(S.big[parity], kNearWide) : S.huges[parity];
@@ -229,54 +235,54 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
                         if (!disc && (f == z || T.last_sq(j) > near_limit(T.E[f] + h))) continue;
                         uint32_t at = 0;
                         if (lane == 0)
-                            at = atomicAdd(disc ? &A.gs->discs[parity] : &A.gs->wides[parity], 1u);
+                            at = atomicAdd(disc ? &put.discs : &put.wides, 1u);
                         at = __shfl_sync(0xffffffffu, at, 0);
                         if (at >= (disc ? A.discs : A.wide))
                             near_far(T, j, z, ~0u, nb.B, nb);  // no room for this one
                         else if (lane == 0)
-                            (disc ? A.gs->disc[parity] : A.gs->wide[parity])[at] = f;
+                            (disc ? A.disc_list + parity * kGridDiscs : A.gs->wide[parity])[at] = f;
                     }
                 }
             }
             // (the clock is slow to read)
             if (tid == 0 && ((sweeps & 15u) == 15u || A.quantum_ns < 1000000u) &&
                 global_timer_ns() - begun > A.quantum_ns)
-                A.gs->pause[parity] = 1u;
+                put.pause = 1u;
             publish(A.gs->keys[parity], nb.key);
             if (!(ok = barrier())) break;
             ++sweeps;
             if (tid == 0) {  // the next sweep's
-                A.gs->wides[parity ^ 1] = A.gs->takers[parity ^ 1] = 0;
-                if (SPREAD) A.gs->discs[parity ^ 1] = 0;
+                auto& next = A.gs->put[parity ^ 1];
+                next.wides = next.discs = next.takers = 0;
             }
             // one warp per CTA reads the keys (all of them reading the same few
             // lines queued up at L2 for 7 us)
             if (warp == 0) {
-                const uint32_t w = *(volatile uint32_t*)&A.gs->wides[parity];
-                const uint32_t d = SPREAD ? *(volatile uint32_t*)&A.gs->discs[parity] : 0u;
-                const uint32_t pause = *(volatile uint32_t*)&A.gs->pause[parity];
+                const uint4 p = __ldcg(reinterpret_cast<const uint4*>(&put));
                 const uint64_t k = near_pick(T, A.gs->keys[parity], ranks, seed);
                 seeds[lane] = make_uint2(seed.a, seed.b);
                 if (lane == 0) {
                     best_key = k;
-                    wide_count = w;
-                    if (SPREAD) disc_count = d;
-                    pause_now = pause;
+                    wide_count = p.x;
+                    pause_now = p.y;
+                    disc_count = p.z;
                 }
             }
             __syncthreads();
             uint64_t key = best_key;
             const uint32_t wides = min(wide_count, A.wide);
             const uint32_t discs = SPREAD ? min(disc_count, A.discs) : 0u;
-            most_wides = max(most_wides, wide_count);
             if (wides || discs) {
+                if (tid == 0) {
+                    most[0] = max(most[0], wide_count);
+                    most[2] = max(most[2], SPREAD ? disc_count : 0u);
+                }
                 const float known = key == kNoMove ? -1.f : (float)key_delta(key);
                 NearBest more{key, known};
                 if constexpr (SPREAD) {
                     // discs put off, a CTA each
-                    most_discs = max(most_discs, disc_count);
                     for (uint32_t d = rank; d < discs; d += ranks) {
-                        const uint32_t j = A.gs->disc[parity][d], jn = T.wrap(j + 1);
+                        const uint32_t j = A.disc_list[parity * kGridDiscs + d], jn = T.wrap(j + 1);
                         const float m =
                             fmaxf(j == z ? kNoEdge : T.E[j], jn == z ? kNoEdge : T.E[jn]);
                         if (2.f * m + 8.f >= -known &&
@@ -294,13 +300,13 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
                         if (votes == 0) continue;
                         uint32_t at = 0;
                         if (lane == 0)
-                            at = atomicAdd(&A.gs->takers[parity], (uint32_t)__popc(votes));
+                            at = atomicAdd(&put.takers, (uint32_t)__popc(votes));
                         at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1u));
                         if (takes && at < A.takers) A.gs->taker[at] = g;
                     }
                     if (!(ok = barrier())) break;
-                    const uint32_t takers = *(volatile uint32_t*)&A.gs->takers[parity];
-                    most_takers = max(most_takers, takers);
+                    const uint32_t takers = *(volatile uint32_t*)&put.takers;
+                    if (tid == 0) most[1] = max(most[1], takers);
                     if (takers <= A.takers) {
                         for (uint32_t base = tid - lane; base < wides * takers; base += threads) {
                             const uint32_t t = base + lane;
@@ -437,9 +443,9 @@ __global__ void __launch_bounds__(kGridNT, 1) near_grid_kernel(GridArgs A) {
             if (bad) atomicOr(&st->status, kErrBadKey);
         }
         st->converged = (step || paused) && ok ? 0u : 1u;
-        A.gs->most_wides = most_wides;
-        A.gs->most_takers = most_takers;
-        A.gs->most_discs = most_discs;
+        A.gs->most_wides = most[0];
+        A.gs->most_takers = most[1];
+        A.gs->most_discs = most[2];
     }
     if (whole) leave();
 }
@@ -464,7 +470,7 @@ int near_grid_ctas(uint32_t n, int device) {
 }
 
 cudaError_t launch_near_grid(const GridArgs& A, bool ils, int ctas, cudaStream_t s) {
-    const cudaError_t e = cudaMemsetAsync(A.gs, 0, offsetof(GridSync, wide_keys), s);
+    const cudaError_t e = cudaMemsetAsync(A.gs, 0, offsetof(GridSync, keys), s);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);

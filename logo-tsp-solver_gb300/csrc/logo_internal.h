@@ -214,23 +214,24 @@ struct GridSync {
     unsigned long long length[2];  // tour length of the descent in hand, by its parity
     unsigned long long start_length;
     unsigned long long bad;        // the route is not a permutation
-    // edges put off in a sweep, and edges that can take part in pairs with them,
-    // by its parity (more may have been offered than fit)
-    uint32_t wides[2], takers[2];
-    uint32_t discs[2];  // slots whose discs are put off, likewise
     uint32_t left;  // CTAs that have left a whole call
-    uint32_t pause[2];  // the launch is to end after this sweep's move, by its parity
+    // by the sweep's parity, read with one load: edges put off, whether the launch is to
+    // end after the sweep's move, slots whose discs are put off; and edges that can take
+    // part in pairs with those put off (more of each may have been offered than fit)
+    struct __align__(16) {
+        uint32_t wides, pause, discs, takers;
+    } put[2];
     // (set to zero up to here before a launch)
-    unsigned long long wide_keys[2][kGridMaxCtas];  // best key per CTA after those
-    uint32_t wide[2][kGridWide];
-    uint32_t disc[2][kGridDiscs];
-    uint32_t taker[kGridTakers];
     unsigned long long keys[2][kGridMaxCtas];  // best key per CTA, by the sweep's parity
+    unsigned long long wide_keys[2][kGridMaxCtas];  // best key per CTA after those put off
+    uint32_t wide[2][kGridWide];
+    uint32_t taker[kGridTakers];
     uint32_t most_wides, most_takers, most_discs;  // largest counts of a sweep of the last launch
 };
 struct GridArgs {
     SoloArgs solo;  // pos: slot of every city meanwhile
     GridSync* gs;
+    uint32_t* disc_list;  // kGridDiscs for each of the two parities
     // limits, at most (a test's are smaller) kGridWide, kGridTakers, kGridDisc, kGridDiscs
     uint32_t wide, takers, disc, discs;
     uint32_t spread;  // tours above as many cities have their large discs dealt to all CTAs
