@@ -5,9 +5,14 @@
 // three times per move (gather + H2D of the ordered coordinates, launch, D2H
 // of best2_out; src/solvers/CUDASolver.cpp:285-386) and applies the move and
 // measures the tour on the host (twoOptLocalSolver.cpp:41-50).  Here the tour
-// stays in HBM: a descent is a CUDA graph of `graph_steps` (sweep, apply)
-// pairs replayed until the device-side convergence flag is set; the host
-// reads one small status block per replay.
+// stays on the device.  By default a best move, a descent or an ILS call is one
+// launch of a cluster (up to 6,144 cities: solo.cu) or launches over the whole
+// device, of 20 ms each (grid_tour.cu), which load the caller's route and leave
+// tour and state in host memory.  Where the caller chose graphs or a sweep kernel,
+// where the search grid tells the cities apart too little, and after a neighbour
+// search's lists in an ILS call, a descent is a CUDA graph of `graph_steps` (sweep,
+// apply) pairs replayed until the device-side convergence flag is set; the host
+// then reads one small status block per replay.
 #include <algorithm>
 #include <cmath>
 #include <condition_variable>

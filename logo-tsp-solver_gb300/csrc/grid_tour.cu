@@ -1,5 +1,5 @@
-// Descents and ILS calls of large tours (n > kSoloMaxN) as one cooperative
-// launch (sm_103a).
+// Descents and ILS calls of large tours (n > kSoloMaxN) as cooperative launches over
+// the whole device (sm_103a).
 //
 // The tour is the ring of near_tour.cuh in global memory (L2: 20 bytes a city);
 // the slots of a sweep are dealt to all warps of the grid, and a move is the
@@ -15,9 +15,12 @@
 // in the state, and the host launches it again behind whatever else is waiting.
 //
 // As a whole call the launch also loads and checks the caller's route and leaves
-// result and state in host memory: one launch and one wait (best move and move
-// of a 100,000-city route: 111 -> 60 us; best move of 1,000,000: 612 -> 168 us,
-// most of it the route's way from host memory).
+// result and state in host memory: one launch and one wait.  Against route load,
+// three sweep kernels and move (us a best move, the other path first): NN tour of
+// n = 6,200 41, 48; 7,000 54, 53; 20,000 70, 55; 40,009 72, 73; 100,000 83, 66; 200,000
+// 132, 86; random tour 65, 42; 79, 42; 45, 49; 46, 59; 58, 66; 84, 75; some hundred
+// moves on 41, 31; 41, 33; 74, 40; 73, 49; 95, 57; 146, 101.  Which of these a caller's
+// route is does not show before the sweep, so no rule of a dispatch chooses.
 //
 // Up to A.spread cities a CTA goes through its large discs itself, above (SPREAD) they
 // are dealt to all CTAs after one more barrier: with more slots a CTA, one had up to

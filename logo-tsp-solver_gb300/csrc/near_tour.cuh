@@ -1,6 +1,7 @@
-// A whole instance held by one CTA (shared memory) and the exact
-// best-improvement sweep over its near neighbours.  Used by the batched solver
-// (batch.cu) and the serving rounds (serve.cu).
+// A tour as a ring of slots and the exact best-improvement sweep over its near
+// neighbours: held by one CTA's shared memory in the batched solver (batch.cu) and
+// the serving rounds (serve.cu), by each CTA of a cluster (solo.cu), and by global
+// memory where the whole device shares it (grid_tour.cu).
 //
 // What bounds it.  A local search is a chain of sweeps, each followed by one
 // move, so a CTA is as fast as one sweep's latency.  Walking all n^2/2 pairs
@@ -42,8 +43,8 @@
 // Positions matter only where the reference lets them: in the tie rule and in
 // the closing edge (n - 1, 0), which is never part of a pair.
 //
-// Shared memory: 51 bytes a city (209 KB at the largest, n = 4,096); the best
-// tour of an iterated search stays in global memory.
+// Shared memory of a CTA that has the lists there too: 51 bytes a city (209 KB at the
+// largest, n = 4,096); the best tour of an iterated search stays in global memory.
 #pragma once
 #include <cstdint>
 

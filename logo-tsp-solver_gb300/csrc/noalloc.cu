@@ -16,7 +16,7 @@
 // delta so far.  B is good before the sweep begins: every window's longest edge
 // is paired with every other's first.  The sweep is bound by the latency of its
 // four dependent launches then, not by the pairs (n = 20,011, clustered, NN tour:
-// 128 -> 58 us; a random tour 191 -> 41; a local optimum 128 -> 73; n = 65,536:
+// 128 -> 51 us; a random tour 191 -> 41; a local optimum 128 -> 73; n = 65,536:
 // 810 -> 72, random 1,320 -> 62; n = 52: 29.5 -> 26.4).
 //
 // Its working memory (the tour-ordered cities, the argmin key, the bounding
