@@ -14,12 +14,14 @@
 // apply) pairs replayed until the device-side convergence flag is set; the host
 // then reads one small status block per replay.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/logo_gpu.h"
@@ -28,6 +30,8 @@
 #include "logo_internal.h"
 
 using namespace logo;
+
+constexpr unsigned long long kCrowdUnknown = ~0ull;
 
 struct logo_ctx {
     int device = 0;
@@ -40,8 +44,8 @@ struct logo_ctx {
     uint32_t* d_route_best = nullptr;
     DevState* d_st = nullptr;
     DevState* h_st = nullptr;  // pinned mirror
-    unsigned long long* h_crowd = nullptr;  // behind it: see launch_near_index
-    mutable bool crowd_known = false;       // (once the lists are built)
+    // behind it: see launch_near_index (kCrowdUnknown until the device has written it)
+    volatile unsigned long long* h_crowd = nullptr;
     uint32_t* d_seen = nullptr;   // route permutation check: last load that met each city
     uint32_t load_epoch = 0;      // loads so far (mod 2^32 - 1, from 1)
     int route_io = LOGO_ROUTE_IO_AUTO;
@@ -762,9 +766,13 @@ bool use_solo(const logo_ctx* c) {
 // and the line with it.
 unsigned long long crowd_most(uint32_t n) { return std::max(100000000ull, 500ull * n); }
 bool crowded(const logo_ctx* c) {
-    if (!c->crowd_known) {
-        if (cudaStreamSynchronize(c->stream) != cudaSuccess) return false;  // (the call says so)
-        c->crowd_known = true;
+    // written by the launches of logo_ctx_create, soon after it: looked at without a
+    // call of the runtime, as the context's stream may be under capture; where other
+    // work holds the device for longer, the answer is no
+    const auto t0 = std::chrono::steady_clock::now();
+    while (*c->h_crowd == kCrowdUnknown) {
+        if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(1)) return false;
+        std::this_thread::yield();
     }
     return *c->h_crowd > crowd_most(c->n);
 }
@@ -1088,6 +1096,7 @@ logo_status logo::create_context(int device, const logo_xy* coords, uint32_t n, 
     CKC(cudaMalloc(&c->d_st, sizeof(DevState)));
     CKC(cudaMallocHost(&c->h_st, sizeof(DevState) + sizeof(unsigned long long)));
     c->h_crowd = reinterpret_cast<unsigned long long*>(c->h_st + 1);
+    *c->h_crowd = kCrowdUnknown;
     CKC(cudaMalloc(&c->d_seen, sizeof(uint32_t) * n));
     // copies and clears go to the context's own stream: it is not ordered with the
     // default stream, on which a copy from pageable memory may still be under way
@@ -1127,7 +1136,8 @@ logo_status logo::create_context(int device, const logo_xy* coords, uint32_t n, 
     c->near.g = near_grid(n, (float)x0, (float)y0, (float)(x1 - x0), (float)(y1 - y0));
     s = rebuild(c);
     if (s != LOGO_OK) return bail(s);
-    CKC(launch_near_index(c->near, c->d_xy, n, c->h_crowd, c->stream));
+    CKC(launch_near_index(c->near, c->d_xy, n, const_cast<unsigned long long*>(c->h_crowd),
+                          c->stream));
 #undef CKC
     *out = c;
     return LOGO_OK;

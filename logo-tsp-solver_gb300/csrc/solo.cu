@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(1024) near_scan_kernel(uint32_t* count, uint32
         cell[cells] = carry;
         for (uint32_t w = 1; w < 32; ++w) mine += squares[w];
         *(volatile unsigned long long*)crowd = mine;
+        __threadfence_system();
     }
 }
 

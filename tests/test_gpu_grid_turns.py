@@ -73,3 +73,31 @@ def test_a_step_does_not_wait_for_another_context(lg, inst):
         t.join()
         assert got == [want] * 3
         assert running and ends["steps"] < ends["ils"]
+
+
+@pytest.mark.parametrize("n", [500, 20000])
+def test_info_leaves_a_capture_alone(lg, inst, oracle_mod, n):
+    """The context's stream may be under capture (logo_enqueue_sweep is a launch
+    like any other): asking for the context's info makes no call on it."""
+    torch = pytest.importorskip("torch")
+    xy = inst.uniform_f32(n, 5, 1.0e5)
+    r = inst.random_tour(n, 6)
+    with lg.Solver(xy) as s:
+        s.set_route(r)
+        s.begin_descent()
+        s.sync()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(torch.cuda.ExternalStream(s.stream)):
+            graph.capture_begin(capture_error_mode="thread_local")
+            grid = s.info()["grid_ctas"]
+            s.enqueue_sweep()
+            s.enqueue_apply()
+            graph.capture_end()
+            graph.replay()
+        assert (grid > 0) == (n > 6144)
+        s.sync()
+        assert s.progress() == (1, False)
+        got = s.get_route()
+    with lg.Solver(xy) as s:
+        want, _ = s.optimize(r, max_moves=1)
+    assert np.array_equal(got, want)
